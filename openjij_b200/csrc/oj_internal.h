@@ -204,6 +204,13 @@ cudaError_t launch_sa_colour(const oj_graph* g, int R, int8_t* spins, const floa
                              int64_t nsweeps, RngBase rb, cudaStream_t st, int* launches);
 cudaError_t launch_sqa_colour(const oj_graph* g, int R, int T, int8_t* spins, const float2* coef,
                               int64_t nsweeps, RngBase rb, cudaStream_t st, int* launches);
+// Small graphs with few sites per colour class (oj_k_seq.cu): the same sweeps
+// as the colour-class kernels, which call them where they apply.
+bool seq_applies(const oj_graph* g, int T);
+cudaError_t launch_sa_seq(const oj_graph* g, int R, int8_t* spins, const float* betas, int64_t nsweeps, RngBase rb,
+                          cudaStream_t st, int* launches);
+cudaError_t launch_sqa_seq(const oj_graph* g, int R, int T, int8_t* spins, const float2* coef, int64_t nsweeps,
+                           RngBase rb, cudaStream_t st, int* launches);
 cudaError_t launch_sa_dense_plain(const oj_graph* g, int R, int8_t* spins, const float* betas,
                                   int64_t nsweeps, RngBase rb, cudaStream_t st, int* launches);
 cudaError_t launch_sa_msc(const oj_graph* g, int G, uint32_t* words, const uint32_t* thr,

@@ -277,6 +277,7 @@ int sa_colour_max_smem_sites() { return kSmemBudget / 4; }
 
 cudaError_t launch_sa_colour(const oj_graph* g, int R, int8_t* spins, const float* betas,
                              int64_t nsweeps, RngBase rb, cudaStream_t st, int* launches) {
+  if (seq_applies(g, 1)) return launch_sa_seq(g, R, spins, betas, nsweeps, rb, st, launches);
   const int quads = (R + 3) / 4;
   const size_t smem = (size_t)4 * g->n;
   const bool use_smem = smem <= (size_t)kSmemBudget;
@@ -300,6 +301,7 @@ cudaError_t launch_sa_colour(const oj_graph* g, int R, int8_t* spins, const floa
 
 cudaError_t launch_sqa_colour(const oj_graph* g, int R, int T, int8_t* spins, const float2* coef,
                               int64_t nsweeps, RngBase rb, cudaStream_t st, int* launches) {
+  if (seq_applies(g, T)) return launch_sqa_seq(g, R, T, spins, coef, nsweeps, rb, st, launches);
   const size_t smem = (size_t)T * g->n;
   const bool use_smem = smem <= (size_t)kSmemBudget;
   if (use_smem) {
