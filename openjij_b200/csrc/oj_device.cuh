@@ -144,6 +144,23 @@ __device__ __forceinline__ float neglog(uint32_t x) {
   return -lnu;
 }
 
+// x - (-ln u) to within kNegLogTol of x - neglog(word), from the hardware
+// logarithm: lg2.approx is within 2^-22 of log2 u for u in (1/2, 1) and within
+// 2^-22 |log2 u| below, |log2 u| <= 24, so the product with ln 2 is within 4e-6
+// of -ln u; neglog is within 6e-8 of it before its last rounding, and that
+// rounding and the two here (values below 17) add at most 3e-6.  A caller
+// accepts where this is negative and calls neglog where its magnitude is not
+// above kNegLogTol: the decisions are those of x < neglog(word), in 5
+// instructions instead of 17.
+constexpr float kNegLogTol = 0x1p-16f;
+
+__device__ __forceinline__ float neglog_gap(float x, uint32_t word) {
+  const float u = __fadd_rn(__uint_as_float(__funnelshift_r(word, 0x7Fu, 9)), -0x1.fffffep-1f);
+  float l;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(u));
+  return __fmaf_rn(l, 0x1.62e430p-1f, x);
+}
+
 // Shared-memory mbarriers and 1-D bulk copies (global -> this CTA's shared
 // memory, no multicast).  Every wait is bounded by an iteration count.
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }

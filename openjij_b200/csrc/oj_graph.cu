@@ -53,6 +53,7 @@ oj_graph::~oj_graph() {
   single.reset();
   single_tab.release();
   sw_tables.release();
+  if (cplan) cplan->tables.release();
   if (msc) msc->tables.release();
   if (tc) {
     tc->bt_hi.release();

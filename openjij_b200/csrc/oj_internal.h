@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -80,6 +81,21 @@ struct MscPlan {
   uint32_t* pent = nullptr;  // [P][pmax]
 };
 
+// Tables of the colour-class kernels.  Slots are the sites in visiting order:
+// by colour class, inside a class by falling degree (a class's sites do not
+// see each other, so their order is free).  A slice is 32 consecutive slots of
+// a class (the last of a class: what is left): its neighbour entries (slot,
+// coupling) are stored term by term, as wide as the slice has slots, up to its
+// largest degree, padded with zero couplings (adding one does not change a sum).
+struct ColourPlan {
+  int ncol = 0, max_class = 0;
+  DevBuf tables;              // one allocation; the pointers below index into it
+  int2* site = nullptr;       // [n] site index, bits of its FP32 field
+  int4* cls = nullptr;        // [ncol] first slot, slots, first slice, 0
+  int2* slice = nullptr;      // [slices] offset of its first entry, terms
+  int2* ent = nullptr;        // neighbour slot, bits of the FP32 coupling
+};
+
 // Launch shape of a tunable kernel; 0 = the kernel's default choice.
 struct Shape {
   int cluster = 0;  // CTAs per thread block cluster
@@ -123,6 +139,10 @@ struct oj_graph {
   std::map<uint64_t, oj::Shape> tuned;  // autotuned launch shapes by (kernel, replicas, slices)
   std::unique_ptr<oj_batch> single;     // this graph as a one-instance batch (dense jump kernel, energies)
   oj::DevBuf single_tab;                // its per-call tables: reads, order, replica and energy offsets
+  // colour-class tables (oj_k_colour.cu), built at the first run; the lock is for
+  // runs of one graph from several threads, each with its own context
+  std::unique_ptr<oj::ColourPlan> cplan;
+  std::mutex cplan_lock;
   int64_t sw_ne = -1;                   // Swendsen-Wang bond count (-1: list not built)
   oj::DevBuf sw_tables;                 // its bond list: i, j, |J|, sign
   ~oj_graph();
@@ -204,6 +224,7 @@ cudaError_t launch_sa_colour(const oj_graph* g, int R, int8_t* spins, const floa
                              int64_t nsweeps, RngBase rb, cudaStream_t st, int* launches);
 cudaError_t launch_sqa_colour(const oj_graph* g, int R, int T, int8_t* spins, const float2* coef,
                               int64_t nsweeps, RngBase rb, cudaStream_t st, int* launches);
+cudaError_t colour_prepare(oj_graph* g);
 // Small graphs with few sites per colour class (oj_k_seq.cu): the same sweeps
 // as the colour-class kernels, which call them where they apply.
 bool seq_applies(const oj_graph* g, int T);

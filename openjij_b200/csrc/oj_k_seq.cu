@@ -410,13 +410,17 @@ cudaError_t launch_seq(const oj_graph* g, int R, int T, int8_t* spins, const flo
 }  // namespace
 
 // A graph goes through the serial kernel when its matrix, spins and uniforms
-// fit shared memory and a sweep is clearly shorter there.  Cycles of a sweep:
-// about n (120 + 1.4 n) here (five sites at once), 1700 + 140 deg per class in
-// the colour-class kernels.  SEQ_RULE
+// fit shared memory and a sweep is shorter there.  Cycles of a sweep: about
+// n (85 + 1.6 n) here (five sites at once), 850 + 55 deg per class in the
+// colour-class kernels.  Measured near the line (SA with 8 replicas, us a sweep
+// there / here): 48 sites, 6 classes of mean degree 10: 4.5 / 3.8; 64 sites, 15
+// classes of degree 32: 17.9 / 6.1; 64 sites, 8 classes of degree 13: 6.2 / 6.1, but
+// with 512 replicas 6.3 / 7.0 (stays there); 100 sites, 11 classes of degree 20:
+// 10.9 / 12.7 (stays there).
 bool seq_applies(const oj_graph* g, int T) {
   const double n = g->n;
   if (g->n < 1 || g->n > kSeqMaxSites || !seq_shape(g->n, T, 1, 1).B) return false;
-  return n * (85.0 + 1.6 * n) < g->info.num_colours * (1700.0 + 140.0 * (double)g->info.nnz / n);
+  return n * (85.0 + 1.6 * n) < 0.95 * g->info.num_colours * (850.0 + 55.0 * (double)g->info.nnz / n);
 }
 
 cudaError_t launch_sa_seq(const oj_graph* g, int R, int8_t* spins, const float* betas, int64_t nsweeps, RngBase rb,
