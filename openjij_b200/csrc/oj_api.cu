@@ -238,7 +238,7 @@ RunCounters read_counters(oj_ctx* ctx) {
 // context; drift and status go to the run counters (armed before).
 oj_status field_call(oj_ctx* ctx, const oj_batch* b, const int32_t* reads, const std::vector<int>& order,
                      int max_reads, FieldCall* fc) {
-  fc->NT = field_tc_tile_replicas(b, max_reads);
+  fc->NT = field_tc_tile_replicas(b, reads, max_reads, ctx->sm_count);
   std::vector<int32_t> it, hot;
   field_tc_items(b, reads, order, fc->NT, it);
   fc->nitems = (int)(it.size() / 3);

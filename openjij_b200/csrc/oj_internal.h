@@ -296,7 +296,7 @@ cudaError_t launch_sa_batch(const oj_batch* b, const int32_t* d_reads, const int
                             int64_t nsweeps, RngBase rb, uint32_t inst0, int sm_count, cudaStream_t st,
                             int* launches, int variant, float* d_fields, const int64_t* d_foff,
                             const FieldCall& fc, double* d_energies = nullptr, const int64_t* d_eoff = nullptr);
-int field_tc_tile_replicas(const oj_batch* b, int max_reads);
+int field_tc_tile_replicas(const oj_batch* b, const int32_t* reads, int max_reads, int sm_count);
 void field_tc_items(const oj_batch* b, const int32_t* reads, const std::vector<int>& order, int NT,
                     std::vector<int32_t>& items);
 cudaError_t launch_field_tc(const oj_batch* b, const int32_t* d_reads, const int64_t* d_soff, const int8_t* spins,

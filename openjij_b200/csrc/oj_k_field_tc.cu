@@ -394,10 +394,21 @@ cudaError_t launch_field_d(const FieldArgs& a, int NT, cudaStream_t st) {
 
 }  // namespace
 
-int field_tc_tile_replicas(const oj_batch* b, int max_reads) {
+// Replicas per tile: as many as a call has reads (up to the tensor-memory
+// columns), the couplings being read once per tile, but no more than leave the
+// SMs a tile each: a call with few instances takes smaller tiles (n = 777, 200
+// reads, four digits: 14 tiles of 128 replicas 74 us, 91 of 16 29 us).
+int field_tc_tile_replicas(const oj_batch* b, const int32_t* reads, int max_reads, int sm_count) {
   const int cap = b->ndig == 1 ? 256 : 128;
+  auto tiles = [&](int nt) {
+    int64_t t = 0;
+    for (int m = 0; m < b->count; ++m)
+      t += ((int64_t)b->n[m] + kChunk - 1) / kChunk * (((int64_t)reads[m] + nt - 1) / nt);
+    return t;
+  };
   int nt = 16;
   while (nt < max_reads && nt < cap) nt *= 2;
+  while (nt > 16 && tiles(nt) < sm_count) nt /= 2;
   return nt;
 }
 
