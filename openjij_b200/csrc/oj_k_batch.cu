@@ -654,12 +654,17 @@ int batch_variant_max_n(int variant) {
   }
 }
 
-int batch_default_variant() {
+// Batches of up to 512 sites (four chunks) take variant 83: a flip row is one
+// group of loads, and more warps hide it.  Larger instances take 45, which has
+// eight chunks' loads in flight: 2048 sites, 4096 replicas, 1000 sweeps 21.9
+// (83), 22.3 (82), 20.0 ms (45); 520 to 2048 sites with 8 to 4096 replicas 2 to 24 %
+// less; 64 instances of 64 to 512 sites with 32 reads 6.4 (83), 7.1 ms (45).
+int batch_default_variant(int max_n) {
   if (const char* env = std::getenv("OJ_BATCH_VARIANT")) {
     const int v = std::atoi(env);
     if (batch_variant_valid(v)) return v;
   }
-  return 83;
+  return max_n > 512 ? 45 : 83;
 }
 
 template <int W, int MINB, int GROUP>
@@ -702,7 +707,7 @@ cudaError_t launch_batch_sweeps(const oj_batch* b, const int32_t* d_reads, const
                                 const int64_t* d_foff, double* d_energies, const int64_t* d_eoff,
                                 bool write_fields, int* d_status, long long wait_limit,
                                 const int32_t* kstart, int recompute, unsigned int* d_drift) {
-  if (variant == 0) variant = batch_default_variant();
+  if (variant == 0) variant = batch_default_variant(b->max_n);
   if (!batch_variant_valid(variant) || b->max_n > batch_variant_max_n(variant)) return cudaErrorInvalidValue;
   if (b->count == 0 || nitems <= 0 || nsweeps <= 0) return cudaSuccess;
   const int fstride = std::max(128, (b->max_n + 127) / 128 * 128);
