@@ -775,7 +775,8 @@ oj_status oj_sa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int8_t* spins, c
           for (int th : {256, 512, 1024}) cand.push_back(Shape{Pc, th, 0});
       int def_msc = -1;  // the heuristic shape
       for (size_t q = 0; q < cand.size(); ++q)
-        if (cand[q].cluster == msc_choose_cluster(g, G, ctx->sm_count) && cand[q].threads == msc_default_threads())
+        if (cand[q].cluster == msc_choose_cluster(g, G, ctx->sm_count) &&
+            cand[q].threads == msc_default_threads(g, cand[q].cluster))
           def_msc = (int)q;
       OJ_CK(ctx->aux.ensure((size_t)G * n * 4), "alloc tuning scratch");
       uint32_t* scratch = ctx->aux.as<uint32_t>();
@@ -797,7 +798,7 @@ oj_status oj_sa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int8_t* spins, c
       tuned_now = true;
     }
     P_used = shp.cluster ? shp.cluster : msc_choose_cluster(g, G, ctx->sm_count);
-    threads_used = shp.threads ? shp.threads : msc_default_threads();
+    threads_used = shp.threads ? shp.threads : msc_default_threads(g, P_used);
     pe = msc_prepare(g, P_used, &why);
     if (pe != cudaSuccess) {
       return prep_fail(ctx, pe, why);

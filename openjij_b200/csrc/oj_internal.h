@@ -346,7 +346,8 @@ cudaError_t launch_best_slice(const double* energies, int R, int T, int32_t* bes
 // Kernel limits used by the planner.
 int sa_colour_max_smem_sites();
 int msc_max_degree();
-int msc_default_threads();
+int msc_default_threads(const oj_graph* g, int P);
+int cluster_most(int G);
 int split_default_threads();
 cudaError_t msc_prepare(oj_graph* g, int P, std::string* why);
 int msc_choose_cluster(const oj_graph* g, int G, int sm_count);

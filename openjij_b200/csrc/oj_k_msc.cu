@@ -50,6 +50,7 @@ constexpr int kMscDefaultThreads = 512;
 constexpr int kMscMaxDegree = 8;
 constexpr int kMscMaxCluster = 16;
 constexpr size_t kMscSmemBytes = 200 * 1024;
+constexpr int kMscDraws = 3;  // Philox calls drawn side by side where latency counts
 
 struct MscArgs {
   const int32_t* gidx;
@@ -91,7 +92,7 @@ struct MscSweep {
 };
 
 template <int D>
-__device__ __forceinline__ MscSweep<D> msc_sweep(const uint32_t* __restrict__ thr_k, uint32_t always_k) {
+__device__ __forceinline__ MscSweep<D> msc_sweep(const uint32_t* thr_k, uint32_t always_k) {
   MscSweep<D> sw;
   sw.alw = 0u;
   sw.live = 0u;
@@ -118,7 +119,9 @@ __device__ __forceinline__ void msc_level(const MscSweep<D>& sw, const uint32_t 
   pending &= ~(pm ^ wl);
 }
 
-template <int D>
+// DR: the first DR Philox calls (4 DR levels) are drawn side by side; the rest one
+// by one while a replica is undecided.
+template <int D, int DR>
 __device__ __forceinline__ uint32_t msc_site(uint32_t w, const uint32_t* __restrict__ Wsh,
                                              const uint16_t* __restrict__ nb, uint32_t jmk,
                                              const MscSweep<D>& sw, uint32_t site, uint32_t sweep,
@@ -153,8 +156,21 @@ __device__ __forceinline__ uint32_t msc_site(uint32_t w, const uint32_t* __restr
   }
   flip |= ~uphill;
   uint32_t lt = 0u;
+  if constexpr (DR > 1) {
+    if (!pending) return w ^ flip;
+    ojd::u4 r[DR];
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
+    for (int q = 0; q < DR; ++q) r[q] = ojd::philox(site, sweep, grp, ((uint32_t)q << 8) | ojd::TAG_SA_MSC, K);
+#pragma unroll
+    for (int q = 0; q < DR; ++q) {
+      msc_level<D>(sw, cls, 31 - 4 * q, r[q].x, pending, lt);
+      msc_level<D>(sw, cls, 30 - 4 * q, r[q].y, pending, lt);
+      msc_level<D>(sw, cls, 29 - 4 * q, r[q].z, pending, lt);
+      msc_level<D>(sw, cls, 28 - 4 * q, r[q].w, pending, lt);
+    }
+  }
+#pragma unroll
+  for (int q = DR > 1 ? DR : 0; q < 8; ++q) {
     if (!pending) break;
     const ojd::u4 r = ojd::philox(site, sweep, grp, ((uint32_t)q << 8) | ojd::TAG_SA_MSC, K);
     msc_level<D>(sw, cls, 31 - 4 * q, r.x, pending, lt);
@@ -166,11 +182,11 @@ __device__ __forceinline__ uint32_t msc_site(uint32_t w, const uint32_t* __restr
 }
 
 // Stores word w of own slot s into the readers' halo slots (boundary slots).
-__device__ __forceinline__ void msc_push(const cg::cluster_group& cl, uint32_t* Wsh, int e0, int e1,
-                                         const uint32_t* __restrict__ pent, uint32_t w) {
+__device__ __forceinline__ void msc_push(uint32_t* Wsh, int e0, int e1, const uint32_t* __restrict__ pent,
+                                         uint32_t w) {
   for (int e = e0; e < e1; ++e) {
     const uint32_t d = __ldg(pent + e);
-    uint32_t* remote = cl.map_shared_rank(Wsh, (int)(d >> 16));
+    uint32_t* remote = cg::this_cluster().map_shared_rank(Wsh, (int)(d >> 16));
     remote[d & 0xFFFFu] = w;
   }
 }
@@ -178,12 +194,11 @@ __device__ __forceinline__ void msc_push(const cg::cluster_group& cl, uint32_t* 
 // Updates own slots [lo, hi), two independent sites per thread and iteration,
 // and pushes the new words of slots >= bnd (the boundary sites) to their
 // readers; returns the number of spins this thread flipped.
-template <int D>
+template <int D, bool CL, int DR>
 __device__ __forceinline__ uint32_t msc_range(int lo, int hi, int bnd, uint32_t* __restrict__ Wsh,
                                               const int32_t* __restrict__ gid, const uint16_t* __restrict__ jm,
                                               const uint16_t* __restrict__ nbr, const int32_t* __restrict__ poff,
-                                              const uint32_t* __restrict__ pent, const cg::cluster_group& cl,
-                                              const MscSweep<D>& sw, uint32_t k, uint32_t g, const ojd::Keys& K) {
+                                              const uint32_t* __restrict__ pent, const MscSweep<D>& sw, uint32_t k, uint32_t g, const ojd::Keys& K) {
   const int T = blockDim.x;
   uint32_t nf = 0u;
   for (int s = lo + threadIdx.x; s < hi; s += 2 * T) {
@@ -192,27 +207,29 @@ __device__ __forceinline__ uint32_t msc_range(int lo, int hi, int bnd, uint32_t*
     // halo stores are in flight while the other site is updated
     if (s2 < hi) {
       const uint32_t w2 = Wsh[s2];
-      const uint32_t b = msc_site<D>(w2, Wsh, nbr + (size_t)s2 * D, jm[s2], sw, (uint32_t)gid[s2], k, g, K);
+      const uint32_t b = msc_site<D, DR>(w2, Wsh, nbr + (size_t)s2 * D, jm[s2], sw, (uint32_t)gid[s2], k, g, K);
       Wsh[s2] = b;
       nf += __popc(b ^ w2);
-      if (s2 >= bnd) msc_push(cl, Wsh, __ldg(poff + s2), __ldg(poff + s2 + 1), pent, b);
+      if (CL && s2 >= bnd) msc_push(Wsh, __ldg(poff + s2), __ldg(poff + s2 + 1), pent, b);
     }
     const uint32_t w0 = Wsh[s];
-    const uint32_t a = msc_site<D>(w0, Wsh, nbr + (size_t)s * D, jm[s], sw, (uint32_t)gid[s], k, g, K);
+    const uint32_t a = msc_site<D, DR>(w0, Wsh, nbr + (size_t)s * D, jm[s], sw, (uint32_t)gid[s], k, g, K);
     Wsh[s] = a;
     nf += __popc(a ^ w0);
-    if (s >= bnd) msc_push(cl, Wsh, __ldg(poff + s), __ldg(poff + s + 1), pent, a);
+    if (CL && s >= bnd) msc_push(Wsh, __ldg(poff + s), __ldg(poff + s + 1), pent, a);
   }
   return nf;
 }
 
 // Shared memory: words[slots] | gid[nlocmax] | jm[nlocmax] | nbr[nlocmax][D]
 // MAXT: the launch bound (512: up to 128 registers a thread; 1024: 64).
-template <int D, int MAXT>
+// CL: the group's sites are split over a cluster of CTAs; without it one CTA
+// owns them all and a phase ends with one block barrier (a cluster phase takes
+// about 1.9 us whatever its work).  DR: see msc_site.
+template <int D, int MAXT, bool CL, int DR>
 __global__ void __launch_bounds__(MAXT) sa_msc_kernel(MscArgs a) {
   extern __shared__ __align__(16) uint32_t Wsh[];
-  cg::cluster_group cl = cg::this_cluster();
-  const int p = (int)cl.block_rank();
+  const int p = CL ? (int)cg::this_cluster().block_rank() : 0;
   const int g = blockIdx.y;
   const int32_t* gid_g = a.gidx + (size_t)p * a.slots;
   const int32_t* co = a.coff + (size_t)p * (a.ncol + 1);
@@ -235,33 +252,45 @@ __global__ void __launch_bounds__(MAXT) sa_msc_kernel(MscArgs a) {
   }
   for (int s = threadIdx.x; s < nloc * D; s += blockDim.x) nbr[s] = nbr_g[s];
   __syncthreads();
-  cluster_arrive();
+  if constexpr (CL) cluster_arrive();
   unsigned long long nflip = 0;
+  MscSweep<D> sw;
+  if (a.nsweeps > 0) sw = msc_sweep<D>(a.thr, a.always[0]);
   for (int64_t k = 0; k < a.nsweeps; ++k) {
-    const MscSweep<D> sw = msc_sweep<D>(a.thr + (size_t)k * (D + 1), a.always[k]);
+    // the next sweep's thresholds are in flight during this one
+    const int64_t kn = k + 1 < a.nsweeps ? k + 1 : k;
+    uint32_t tn[D + 1];
+#pragma unroll
+    for (int u = 0; u <= D; ++u) tn[u] = __ldg(a.thr + (size_t)kn * (D + 1) + u);
+    const uint32_t an = __ldg(a.always + kn);
     const uint32_t kk = a.sweep0 + (uint32_t)k, gg = a.group0 + (uint32_t)g;
     for (int c = 0; c < a.ncol; ++c) {
-      // the class's sites go in rounds of 2 x blockDim.x (two per thread):
-      // the interior sites of all rounds but the last run before the cluster
-      // wait, the rest of the interior with the boundary sites after the halo
-      // refresh, so that no round is left to the few boundary sites alone
-      // (sites of one class do not read each other: any order gives the same
-      // words)
-      const int step = 2 * (int)blockDim.x, nc = co[c + 1] - co[c];
-      const int split = co[c] + min(cb[c] - co[c], max(0, (nc + step - 1) / step * step - step));
-      nflip += msc_range<D>(co[c], split, cb[c], Wsh, gid, jm, nbr, poff, pent, cl, sw, kk, gg, a.keys);
-      // after the wait every halo word this class reads has been pushed (the
-      // same-class sites of this round do not read each other)
-      cluster_wait();
-      nflip += msc_range<D>(split, co[c + 1], cb[c], Wsh, gid, jm, nbr, poff, pent, cl, sw, kk, gg, a.keys);
-      // arrive first (its release covers this thread's halo stores), then the
-      // CTA barrier (the next phase reads this phase's words of other
-      // threads); the other order measured slower
-      cluster_arrive();
+      if constexpr (CL) {
+        // the class's sites go in rounds of 2 x blockDim.x (two per thread):
+        // the interior sites of all rounds but the last run before the cluster
+        // wait, the rest of the interior with the boundary sites after the halo
+        // refresh, so that no round is left to the few boundary sites alone
+        // (sites of one class do not read each other: any order gives the same
+        // words)
+        const int step = 2 * (int)blockDim.x, nc = co[c + 1] - co[c];
+        const int split = co[c] + min(cb[c] - co[c], max(0, (nc + step - 1) / step * step - step));
+        nflip += msc_range<D, CL, DR>(co[c], split, cb[c], Wsh, gid, jm, nbr, poff, pent, sw, kk, gg, a.keys);
+        // after the wait every halo word this class reads has been pushed (the
+        // same-class sites of this round do not read each other)
+        cluster_wait();
+        nflip += msc_range<D, CL, DR>(split, co[c + 1], cb[c], Wsh, gid, jm, nbr, poff, pent, sw, kk, gg, a.keys);
+        // arrive first (its release covers this thread's halo stores), then the
+        // CTA barrier (the next phase reads this phase's words of other
+        // threads); the other order measured slower
+        cluster_arrive();
+      } else {
+        nflip += msc_range<D, CL, DR>(co[c], co[c + 1], 0, Wsh, gid, jm, nbr, poff, pent, sw, kk, gg, a.keys);
+      }
       __syncthreads();
     }
+    sw = msc_sweep<D>(tn, an);
   }
-  cluster_wait();
+  if constexpr (CL) cluster_wait();
   for (int s = threadIdx.x; s < nloc; s += blockDim.x) gw[gid[s]] = Wsh[s];
   ojd::add_flips(a.flips, nflip);
 }
@@ -270,21 +299,33 @@ size_t msc_smem_bytes(const MscPlan& pl) {
   return (size_t)pl.slots * 4 + (size_t)pl.nlocmax * (4 + 2 + 2 * pl.D) + 16;
 }
 
-int msc_threads() {
-  int threads = kMscDefaultThreads;
-  if (const char* env = std::getenv("OJ_MSC_THREADS")) {
-    const int v = std::atoi(env);
-    if (v >= 32 && v <= kMscMaxThreads && v % 32 == 0) threads = v;
-  }
-  return threads;
+// Sites of the largest colour class.
+int largest_class(const oj_graph* g) {
+  int m = 1;
+  for (size_t c = 0; c + 1 < g->coff.size(); ++c) m = std::max(m, g->coff[c + 1] - g->coff[c]);
+  return m;
 }
 
+// A thread with at most two sites of a class is bound by the latency of their
+// draws, which then go side by side (lattice of 33 x 33, 1000 sweeps, one CTA per
+// group: 6.5 ms drawn one by one, 4.34 ms); with more sites a thread the draws that
+// a decided site would not have taken cost more (128 x 128 on 4 CTAs).
 template <int D>
 cudaError_t launch_d(const MscPlan& pl, const MscArgs& a, int G, cudaStream_t st, int threads) {
-  auto kern = threads <= 512 ? sa_msc_kernel<D, 512> : sa_msc_kernel<D, kMscMaxThreads>;
+  const int per_class = (pl.nlocmax + pl.ncol - 1) / pl.ncol;
+  const bool latency = threads <= 512 && per_class <= 2 * threads;
+  const bool single = pl.P == 1 && (latency || threads > 512);
+  auto kern = threads > 512 ? (single ? sa_msc_kernel<D, kMscMaxThreads, false, 1> : sa_msc_kernel<D, kMscMaxThreads, true, 1>)
+                            : (!latency ? sa_msc_kernel<D, 512, true, 1>
+                                        : (pl.P > 1 ? sa_msc_kernel<D, 512, true, kMscDraws>
+                                                    : sa_msc_kernel<D, 512, false, kMscDraws>));
   const size_t smem = msc_smem_bytes(pl);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
+  if (single) {
+    kern<<<dim3(1, G, 1), threads, smem, st>>>(a);
+    return cudaGetLastError();
+  }
   if (pl.P > 8) {
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
@@ -311,26 +352,56 @@ int msc_max_degree() { return kMscMaxDegree; }
 cudaError_t msc_preload() {
   cudaFuncAttributes fa;
   cudaError_t e = cudaSuccess;
-  auto load = [&](auto k512, auto k1024) {
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k512);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k1024);
+  auto load = [&](auto... kern) {
+    ((e = e == cudaSuccess ? cudaFuncGetAttributes(&fa, kern) : e), ...);
   };
-  load(sa_msc_kernel<1, 512>, sa_msc_kernel<1, kMscMaxThreads>);
-  load(sa_msc_kernel<2, 512>, sa_msc_kernel<2, kMscMaxThreads>);
-  load(sa_msc_kernel<3, 512>, sa_msc_kernel<3, kMscMaxThreads>);
-  load(sa_msc_kernel<4, 512>, sa_msc_kernel<4, kMscMaxThreads>);
-  load(sa_msc_kernel<5, 512>, sa_msc_kernel<5, kMscMaxThreads>);
-  load(sa_msc_kernel<6, 512>, sa_msc_kernel<6, kMscMaxThreads>);
-  load(sa_msc_kernel<7, 512>, sa_msc_kernel<7, kMscMaxThreads>);
-  load(sa_msc_kernel<8, 512>, sa_msc_kernel<8, kMscMaxThreads>);
+  auto load_d = [&](auto d) {
+    constexpr int D = decltype(d)::value;
+    load(sa_msc_kernel<D, 512, true, 1>, sa_msc_kernel<D, kMscMaxThreads, true, 1>,
+         sa_msc_kernel<D, kMscMaxThreads, false, 1>,
+         sa_msc_kernel<D, 512, true, kMscDraws>, sa_msc_kernel<D, 512, false, kMscDraws>);
+  };
+  load_d(std::integral_constant<int, 1>());
+  load_d(std::integral_constant<int, 2>());
+  load_d(std::integral_constant<int, 3>());
+  load_d(std::integral_constant<int, 4>());
+  load_d(std::integral_constant<int, 5>());
+  load_d(std::integral_constant<int, 6>());
+  load_d(std::integral_constant<int, 7>());
+  load_d(std::integral_constant<int, 8>());
   return e;
 }
-int msc_default_threads() { return msc_threads(); }
+
+// Threads of a CTA: a whole group in one CTA takes one per site of its largest
+// class (8 x 8 lattice: 512 threads 1.46 us a sweep, 64 1.33); a cluster 256 up to
+// two sites a thread (128 x 128 on 16 CTAs: 512 threads 5.15 us, 256 4.84), else 512.
+int msc_default_threads(const oj_graph* g, int P) {
+  if (const char* env = std::getenv("OJ_MSC_THREADS")) {
+    const int v = std::atoi(env);
+    if (v >= 32 && v <= kMscMaxThreads && v % 32 == 0) return v;
+  }
+  const int per = (largest_class(g) + P - 1) / P;
+  if (P == 1) return std::max(64, std::min(kMscDefaultThreads, (per + 31) / 32 * 32));
+  return per <= 512 ? 256 : kMscDefaultThreads;
+}
+
+// The most CTAs a cluster may have for G clusters to run at once: a cluster
+// stays within a GPC, of which a B200 has eight with at least 18 SMs (13 groups of
+// a 128 x 128 lattice: 11 CTAs a cluster, eight clusters at a time, 8.8 us a sweep;
+// 8 CTAs, all at once, 6.3 us).
+int cluster_most(int G) {
+  constexpr int kGpcs = 8, kGpcSms = 18, kMost = 16;
+  int P = kMost;
+  while (P > 1 && kGpcSms / P * kGpcs < G) --P;
+  return P;
+}
 
 // Cluster size: the number of CTAs per replica group.  One CTA per SM, as
-// many CTAs as fit on the SMs (measured on the L=128 lattice: one 512-thread
+// many CTAs as run at once (measured on the L=128 lattice: one 512-thread
 // CTA per SM beats two smaller ones and uneven multi-CTA packings), within the
-// shared-memory budget and the 16-CTA non-portable cluster limit.
+// shared-memory budget; a single CTA, whose phases need no cluster barrier, up to
+// 640 sites a class (us a sweep with one CTA / a cluster, 32 replicas: 45 x 45, four
+// classes of 507 sites, 5.7 / 7.4; 36 x 36, two of 648, 4.0 / 3.7).
 int msc_choose_cluster(const oj_graph* g, int G, int sm_count) {
   if (const char* env = std::getenv("OJ_MSC_CLUSTER")) {
     const int v = std::atoi(env);
@@ -341,8 +412,9 @@ int msc_choose_cluster(const oj_graph* g, int G, int sm_count) {
     const size_t per = (size_t)((g->n + P - 1) / P);
     return per * (4 + 6 + 2 * (size_t)D) + per / 2 * 4 <= kMscSmemBytes;
   };
-  int P = std::max(1, std::min(kMscMaxCluster, sm_count / std::max(G, 1)));
+  int P = std::max(1, std::min(cluster_most(G), sm_count / std::max(G, 1)));
   while (P > 1 && g->n / P < 256) --P;
+  if (largest_class(g) <= 640) P = 1;
   while (P < kMscMaxCluster && !fits(P)) ++P;
   return P;
 }
@@ -512,7 +584,7 @@ cudaError_t msc_prepare(oj_graph* g, int P, std::string* why) {
 cudaError_t launch_sa_msc(const oj_graph* g, int G, uint32_t* words, const uint32_t* thr,
                           const uint32_t* always, int64_t nsweeps, RngBase rb, cudaStream_t st,
                           int* launches, int threads) {
-  if (threads == 0) threads = msc_threads();
+  if (threads == 0) threads = msc_default_threads(g, g->msc->P);
   if (threads < 32 || threads > kMscMaxThreads || threads % 32) return cudaErrorInvalidValue;
   const MscPlan& pl = *g->msc;
   MscArgs a;
