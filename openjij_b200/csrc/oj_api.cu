@@ -1807,7 +1807,7 @@ oj_status oj_sw_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int8_t* spins, c
     OJ_CK(ctx->aux.ensure(per * (size_t)chunk), "alloc union-find scratch");
     scratch = ctx->aux.as<uint32_t>();
   }
-  if (S > 0) OJ_CK(launch_sw(g, R, d_spins, d_beta, S, rb, scratch, chunk, st, &launches), "swendsen-wang kernel");
+  if (S > 0) OJ_CK(launch_sw(g, R, d_spins, d_beta, S, rb, scratch, chunk, ctx->sm_count, st, &launches), "swendsen-wang kernel");
   OJ_CK(cudaEventRecord(ctx->ev[2], st), "event");
   if (energies) {
     double* d_e = energies;
@@ -1826,7 +1826,7 @@ oj_status oj_sw_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int8_t* spins, c
     stats->launches = launches;
     stats->sweeps = S;
     stats->attempts = (double)R * n * (double)S;
-    stats->threads = 512;
+    stats->threads = sw_threads(g, R, ctx->sm_count);
     stats->accepted = -1.0;
     stats->field_drift = -1.0;
     cudaEventElapsedTime(&stats->anneal_ms, ctx->ev[1], ctx->ev[2]);

@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "oj_device.cuh"
@@ -36,13 +37,16 @@ namespace oj {
 namespace {
 
 constexpr int kSwThreads = 512;
+constexpr int kSwHookThreads = 1024;  // most threads of the hooking kernel
+constexpr size_t kSwHookSmemBytes = 220 * 1024;
 
 struct SwArgs {
   const int32_t* ei;   // [ne] bond endpoints, ei < ej (ej == n: the dummy spin)
   const int32_t* ej;
   const float* w;      // [ne] |J| of the bond (FP32)
   const uint8_t* pos;  // [ne] 1 when J > 0
-  int ne, n;
+  const int4* quad;    // [nq][2] four bonds: ei | ej << 16, J (FP32 bits), padded with J = 0
+  int ne, n, nq;
   int8_t* spins;       // [R][n]
   const float* betas;  // [nsweeps]
   int64_t nsweeps;
@@ -88,6 +92,156 @@ __device__ __forceinline__ void unite(uint32_t* parent, uint32_t a, uint32_t b) 
     // hook the larger root under the smaller; retry if a moved meanwhile
     if (atomicCAS(&parent[a], a, b) == a) return;
   }
+}
+
+// Large graphs, and calls with few replicas (sw_hooks).  What bounds sw_kernel there
+// is the serial chains of its unions: lanes walk to their roots and retry at
+// different lengths.  Here no lane walks: a pass hooks the larger root of every kept
+// bond between two trees under the smaller with one atomic minimum, then all links
+// jump to their roots together; passes go on until no kept bond joins two trees.  The
+// coins are drawn four a Philox call, spins are bits, a bond is one 8-byte entry,
+// and the kept test takes the hardware logarithm first (neglog_gap).  One CTA per
+// replica.  Shared memory: parent[n + 1] | spin bits | coin bits | kept bonds.
+// Measured (us a sweep, sw_kernel / this one): lattice 128 x 128, 16 replicas 97 / 44,
+// 1024 replicas 419 / 300; lattice 64 x 64, 16 replicas 19.1 / 13.0, but 256 replicas
+// 23.8 / 23.3 and 1024 replicas 65.4 / 67.3; Chimera 16 x 16 cells with fields, 16
+// replicas 18.3 / 10.2, 256 replicas 22.2 / 17.9.
+template <int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) sw_hook_kernel(SwArgs a) {
+  extern __shared__ __align__(16) uint32_t parent[];
+  __shared__ uint32_t dummy_root;
+  const int n = a.n, T = blockDim.x, nw = (n + 32) >> 5;
+  uint32_t* sb = parent + n + 1;
+  uint32_t* coin = sb + nw;
+  uint8_t* kept = reinterpret_cast<uint8_t*>(coin + nw);  // four bits per quad
+  const int r = blockIdx.x, lane = threadIdx.x & 31, base = threadIdx.x - lane;
+  int8_t* gs = a.spins + (size_t)r * n;
+  for (int x0 = base; x0 <= n; x0 += T) {  // whole warps: x0 a multiple of 32
+    const int x = x0 + lane;
+    const uint32_t w = __ballot_sync(0xffffffffu, x < n && gs[x] < 0);
+    if (lane == 0) sb[x0 >> 5] = w;
+    if (x <= n) parent[x] = (uint32_t)x;
+  }
+  __syncthreads();
+  const uint32_t rg = a.rep0 + (uint32_t)r;
+  float bnext = a.nsweeps > 0 ? __ldg(a.betas) : 0.0f;
+  for (int64_t k = 0; k < a.nsweeps; ++k) {
+    const float beta2 = __fmul_rn(2.0f, bnext);
+    if (k + 1 < a.nsweeps) bnext = __ldg(a.betas + k + 1);
+    const uint32_t kk = a.sweep0 + (uint32_t)k;
+    // 1. bonds, four per thread and Philox call; a kept bond hooks its larger
+    // end under its smaller one unless that has a smaller parent already
+    uint32_t low = (uint32_t)n;  // the dummy spin's smallest kept neighbour
+    for (int q0 = base; q0 < a.nq; q0 += T) {
+      const int q = q0 + lane;
+      uint32_t nib = 0u;
+      if (q < a.nq) {
+        const int4 b0 = __ldg(a.quad + 2 * q), b1 = __ldg(a.quad + 2 * q + 1);
+        const ojd::u4 u = ojd::philox((uint32_t)q, kk, rg, ojd::TAG_SW_BOND, a.keys);
+        const uint32_t ends[4] = {(uint32_t)b0.x, (uint32_t)b0.z, (uint32_t)b1.x, (uint32_t)b1.z};
+        const uint32_t js[4] = {(uint32_t)b0.y, (uint32_t)b0.w, (uint32_t)b1.y, (uint32_t)b1.w};
+        bool near = false;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t i = ends[e] & 0xFFFFu, j = ends[e] >> 16;
+          // bit 0: satisfied (J s_i s_j < 0); the dummy spin is +1
+          const uint32_t sat = (sb[i >> 5] >> (i & 31u)) ^ (sb[j >> 5] >> (j & 31u)) ^ (js[e] >> 31);
+          const float y = __fmul_rn(beta2, __uint_as_float(js[e] & 0x7FFFFFFFu));
+          const float t = ojd::neglog_gap(y, ojd::pick(u, e));  // 2 beta |J| - (-ln u)
+          near = near || fabsf(t) <= ojd::kNegLogTol;
+          if ((sat & 1u) && t > 0.0f) nib |= 1u << e;
+        }
+        if (near) {
+          nib = 0u;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const uint32_t i = ends[e] & 0xFFFFu, j = ends[e] >> 16;
+            const uint32_t sat = (sb[i >> 5] >> (i & 31u)) ^ (sb[j >> 5] >> (j & 31u)) ^ (js[e] >> 31);
+            if ((sat & 1u) && ojd::neglog(ojd::pick(u, e)) < __fmul_rn(beta2, __uint_as_float(js[e] & 0x7FFFFFFFu)))
+              nib |= 1u << e;
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t i = ends[e] & 0xFFFFu, j = ends[e] >> 16;
+          if ((nib >> e) & 1u) {
+            if (j < (uint32_t)n) atomicMin(parent + j, i);
+            else low = min(low, i);
+          }
+        }
+      }
+      if (q < a.nq) kept[q] = (uint8_t)nib;
+    }
+    low = __reduce_min_sync(0xffffffffu, low);
+    if (lane == 0 && low < (uint32_t)n) atomicMin(parent + n, low);
+    __syncthreads();
+    // the coins of all sites, four per Philox call (a root's is read)
+    for (int q0 = base; 4 * q0 < n; q0 += T) {
+      const ojd::u4 c = ojd::philox((uint32_t)(q0 + lane), kk, rg, ojd::TAG_SW_FLIP, a.keys);
+      uint32_t nib = ((c.x & 1u) | ((c.y & 1u) << 1) | ((c.z & 1u) << 2) | ((c.w & 1u) << 3)) << (4 * (lane & 7));
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) nib |= __shfl_xor_sync(0xffffffffu, nib, o);
+      if ((lane & 7) == 0 && 4 * (q0 + lane) <= n) coin[(q0 + lane) >> 3] = nib;
+    }
+    // 2. passes until every kept bond has both ends under one root: flatten the
+    // trees (every site's link moves up to four steps a round until it is a
+    // root), then every kept bond between two trees hooks the larger root under
+    // the smaller and stays in the list, the others leave it.  A hook that loses
+    // to a smaller one in the same pass is made again in the next, as its bond
+    // is still listed.
+    bool hooked = true;
+    while (__syncthreads_or(hooked)) {
+      hooked = false;
+      bool more = true;
+      while (__syncthreads_or(more)) {
+        more = false;
+        for (int x = threadIdx.x; x <= n; x += T) {
+          const uint32_t p0 = parent[x];
+          uint32_t p = p0;
+          bool up = true;
+#pragma unroll
+          for (int h = 0; h < 4 && up; ++h) {
+            const uint32_t g = parent[p];
+            up = g != p;
+            p = g;
+          }
+          if (p != p0) parent[x] = p;
+          more = more || up;
+        }
+      }
+      for (int q = threadIdx.x; q < a.nq; q += T) {
+        uint32_t nib = kept[q];
+        if (!nib) continue;
+        const int4 b0 = __ldg(a.quad + 2 * q), b1 = __ldg(a.quad + 2 * q + 1);
+        const uint32_t ends[4] = {(uint32_t)b0.x, (uint32_t)b0.z, (uint32_t)b1.x, (uint32_t)b1.z};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t ri = parent[ends[e] & 0xFFFFu], rj = parent[ends[e] >> 16];
+          if (ri == rj) nib &= ~(1u << e);
+          if ((nib >> e) & 1u) atomicMin(parent + max(ri, rj), min(ri, rj));
+        }
+        kept[q] = (uint8_t)nib;
+        hooked = hooked || nib;
+      }
+    }
+    // 3. (the last pass hooked nothing: every link is a root)
+    if (threadIdx.x == 0) dummy_root = parent[n];
+    __syncthreads();
+    const uint32_t rn = dummy_root;
+    for (int x0 = base; x0 <= n; x0 += T) {
+      const int x = x0 + lane;
+      bool flip = false;
+      if (x <= n) {
+        const uint32_t root = parent[x];
+        flip = x < n && root != rn && ((coin[root >> 5] >> (root & 31u)) & 1u);
+        parent[x] = (uint32_t)x;  // for the next sweep
+      }
+      const uint32_t w = __ballot_sync(0xffffffffu, flip);
+      if (lane == 0) sb[x0 >> 5] ^= w;
+    }
+    __syncthreads();
+  }
+  for (int x = threadIdx.x; x < n; x += T) gs[x] = ((sb[x >> 5] >> (x & 31)) & 1u) ? (int8_t)-1 : (int8_t)1;
 }
 
 // SMEM: shared memory holds parent[n + 1] (u32) | spins[n] (int8).  Otherwise
@@ -142,6 +296,32 @@ __global__ void __launch_bounds__(kSwThreads) sw_kernel(SwArgs a, uint32_t* gpar
 
 size_t sw_smem_bytes(int n) { return (size_t)(n + 1) * 4 + (size_t)n + 16; }
 
+namespace {
+
+size_t sw_align(size_t b) { return (b + 255) & ~(size_t)255; }
+
+// Shared memory of sw_hook_kernel: parent links, spin and coin bits, kept bonds.
+size_t sw_hook_smem(int n, size_t nq) { return 4 * ((size_t)(n + 1) + 2 * ((size_t)(n + 32) / 32)) + (nq + 3) / 4 * 4; }
+
+// Bytes of the separate bond arrays; the quads follow them.
+size_t sw_array_bytes(size_t ne) { return 2 * sw_align(ne * 4 + 4) + sw_align(ne * 4 + 4) + sw_align(ne + 1); }
+
+// The graph has quads: its sites are 16-bit indices and its state fits.
+bool sw_has_quads(int n, size_t ne) { return n < 65535 && sw_hook_smem(n, (ne + 3) / 4) <= kSwHookSmemBytes; }
+
+// The hooking kernel (figures there) from 8192 sites on, from 2048 on with at most two
+// replicas an SM, and from 1024 on where every replica has an SM to itself (1024
+// threads each).
+bool sw_hooks(const oj_graph* g, int R, int sm_count) {
+  return sw_has_quads(g->n, (size_t)g->sw_ne) && (g->n >= 8192 || (g->n >= 2048 && R <= 2 * sm_count) || (g->n >= 1024 && R <= sm_count));
+}
+
+}  // namespace
+
+int sw_threads(const oj_graph* g, int R, int sm_count) {
+  return sw_hooks(g, R, sm_count) && R <= sm_count ? kSwHookThreads : kSwThreads;
+}
+
 // Bond list of the graph: (i, j) with i < j from the neighbour lists, then
 // (i, n) for every non-zero h_i; built once per graph.
 cudaError_t sw_prepare(oj_graph* g) {
@@ -166,11 +346,22 @@ cudaError_t sw_prepare(oj_graph* g) {
       pos.push_back(g->h64[i] > 0 ? 1 : 0);
     }
   const size_t ne = ei.size();
-  auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const size_t b_i = al(ne * 4 + 4), b_w = al(ne * 4 + 4), b_p = al(ne + 1);
-  cudaError_t e = g->sw_tables.ensure(2 * b_i + b_w + b_p);
+  const size_t b_i = sw_align(ne * 4 + 4), b_w = sw_align(ne * 4 + 4), nq = (ne + 3) / 4;
+  const bool quads = sw_has_quads(g->n, ne);
+  cudaError_t e = g->sw_tables.ensure(sw_array_bytes(ne) + (quads ? 32 * nq : 0));
   if (e != cudaSuccess) return e;
   char* base = g->sw_tables.as<char>();
+  if (quads && ne) {
+    std::vector<uint32_t> quad(8 * nq, 0u);
+    for (size_t b = 0; b < ne; ++b) {
+      uint32_t bits;
+      std::memcpy(&bits, &w[b], 4);
+      quad[2 * b] = (uint32_t)ei[b] | ((uint32_t)ej[b] << 16);
+      quad[2 * b + 1] = bits | (pos[b] ? 0u : 0x80000000u);
+    }
+    e = cudaMemcpy(base + sw_array_bytes(ne), quad.data(), quad.size() * 4, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return e;
+  }
   if (ne) {
     if ((e = cudaMemcpy(base, ei.data(), ne * 4, cudaMemcpyHostToDevice)) != cudaSuccess) return e;
     if ((e = cudaMemcpy(base + b_i, ej.data(), ne * 4, cudaMemcpyHostToDevice)) != cudaSuccess) return e;
@@ -182,20 +373,21 @@ cudaError_t sw_prepare(oj_graph* g) {
 }
 
 cudaError_t launch_sw(const oj_graph* g, int R, int8_t* spins, const float* betas, int64_t nsweeps, RngBase rb,
-                      uint32_t* scratch, int chunk, cudaStream_t st, int* launches) {
+                      uint32_t* scratch, int chunk, int sm_count, cudaStream_t st, int* launches) {
   const int n = g->n;
   const bool in_smem = n <= sw_max_sites();
   const size_t smem = in_smem ? sw_smem_bytes(n) : 0;
   if (g->sw_ne > (int64_t)0x7FFFFFFF || (!in_smem && (!scratch || chunk < 1))) return cudaErrorInvalidValue;
   const int64_t ne = g->sw_ne;
-  auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const size_t b_i = al((size_t)ne * 4 + 4), b_w = al((size_t)ne * 4 + 4);
+  const size_t b_i = sw_align((size_t)ne * 4 + 4), b_w = sw_align((size_t)ne * 4 + 4);
   const char* base = g->sw_tables.as<char>();
   SwArgs a;
   a.ei = reinterpret_cast<const int32_t*>(base);
   a.ej = reinterpret_cast<const int32_t*>(base + b_i);
   a.w = reinterpret_cast<const float*>(base + 2 * b_i);
   a.pos = reinterpret_cast<const uint8_t*>(base + 2 * b_i + b_w);
+  a.quad = reinterpret_cast<const int4*>(base + sw_array_bytes((size_t)ne));
+  a.nq = (int)((ne + 3) / 4);
   a.ne = (int)ne;
   a.n = n;
   a.spins = spins;
@@ -204,6 +396,16 @@ cudaError_t launch_sw(const oj_graph* g, int R, int8_t* spins, const float* beta
   a.keys = ojd::make_keys(rb.k0, rb.k1);
   a.sweep0 = rb.sweep0;
   a.rep0 = rb.rep0;
+  if (sw_hooks(g, R, sm_count)) {
+    const int threads = sw_threads(g, R, sm_count);
+    auto kern = threads > kSwThreads ? sw_hook_kernel<kSwHookThreads, 1> : sw_hook_kernel<kSwThreads, 4>;
+    const size_t hook_smem = sw_hook_smem(n, (size_t)a.nq);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hook_smem);
+    if (e != cudaSuccess) return e;
+    kern<<<R, threads, hook_smem, st>>>(a);
+    if (launches) ++*launches;
+    return cudaGetLastError();
+  }
   if (in_smem) {
     cudaError_t e = cudaFuncSetAttribute(sw_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
