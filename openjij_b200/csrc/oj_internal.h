@@ -349,7 +349,8 @@ int sa_colour_max_smem_sites();
 int msc_max_degree();
 int msc_default_threads(const oj_graph* g, int P);
 int cluster_most(int G);
-int split_default_threads();
+int split_default_threads(const oj_graph* g, int P);
+int largest_class(const oj_graph* g);
 cudaError_t msc_prepare(oj_graph* g, int P, std::string* why);
 int msc_choose_cluster(const oj_graph* g, int G, int sm_count);
 

@@ -299,13 +299,6 @@ size_t msc_smem_bytes(const MscPlan& pl) {
   return (size_t)pl.slots * 4 + (size_t)pl.nlocmax * (4 + 2 + 2 * pl.D) + 16;
 }
 
-// Sites of the largest colour class.
-int largest_class(const oj_graph* g) {
-  int m = 1;
-  for (size_t c = 0; c + 1 < g->coff.size(); ++c) m = std::max(m, g->coff[c + 1] - g->coff[c]);
-  return m;
-}
-
 // A thread with at most two sites of a class is bound by the latency of their
 // draws, which then go side by side (lattice of 33 x 33, 1000 sweeps, one CTA per
 // group: 6.5 ms drawn one by one, 4.34 ms); with more sites a thread the draws that
@@ -372,8 +365,16 @@ cudaError_t msc_preload() {
   return e;
 }
 
+// Sites of the largest colour class.
+int largest_class(const oj_graph* g) {
+  int m = 1;
+  for (size_t c = 0; c + 1 < g->coff.size(); ++c) m = std::max(m, g->coff[c + 1] - g->coff[c]);
+  return m;
+}
+
 // Threads of a CTA: a whole group in one CTA takes one per site of its largest
-// class (8 x 8 lattice: 512 threads 1.46 us a sweep, 64 1.33); a cluster 256 up to
+// class (8 x 8 lattice: 512 threads 1.46 us a sweep, 64 1.33), above 1024 sites 1024
+// (100 x 100, 4096 replicas: 512 threads 21.8 us, 1024 20.6); a cluster 256 up to
 // two sites a thread (128 x 128 on 16 CTAs: 512 threads 5.15 us, 256 4.84), else 512.
 int msc_default_threads(const oj_graph* g, int P) {
   if (const char* env = std::getenv("OJ_MSC_THREADS")) {
@@ -381,6 +382,7 @@ int msc_default_threads(const oj_graph* g, int P) {
     if (v >= 32 && v <= kMscMaxThreads && v % 32 == 0) return v;
   }
   const int per = (largest_class(g) + P - 1) / P;
+  if (P == 1 && per > 1024) return kMscMaxThreads;
   if (P == 1) return std::max(64, std::min(kMscDefaultThreads, (per + 31) / 32 * 32));
   return per <= 512 ? 256 : kMscDefaultThreads;
 }

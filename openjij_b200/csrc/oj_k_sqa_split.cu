@@ -41,6 +41,11 @@ namespace {
 constexpr int kSplitMaxThreads = 512;
 constexpr int kSplitDefaultThreads = 512;
 constexpr int kSplitMaxCluster = 16;
+// Philox calls drawn side by side by a CTA with a whole group (3-regular, us a sweep
+// one by one / side by side: 70 sites 5.68 / 5.15, 4096 sites, T = 32, 256 replicas 23.2 /
+// 22.5); in a cluster they only lengthen the work between its barriers (4096 sites,
+// T = 16, 8 replicas: 16.7 / 20.1).
+constexpr int kSplitDraws = 3;
 constexpr size_t kSplitSmemBytes = 200 * 1024;
 
 struct SplitArgs {
@@ -163,7 +168,9 @@ __device__ __forceinline__ uint32_t tab_eval_dominated(const uint32_t* __restric
 
 // New value of word x (half q) of one site: nb are the neighbour slots in X
 // (the array being updated), y the site's other half, tab the sweep's tables.
-template <int D, bool DOM>
+// DR: the first DR Philox calls are drawn side by side, the rest one by one while
+// a bit is undecided.
+template <int D, bool DOM, int DR>
 __device__ __forceinline__ uint32_t split_site(uint32_t x, const uint32_t* __restrict__ X,
                                                const uint16_t* __restrict__ nb, uint32_t jmk, uint32_t y,
                                                int q, const SplitArgs& a, const uint32_t* __restrict__ tab,
@@ -191,11 +198,10 @@ __device__ __forceinline__ uint32_t split_site(uint32_t x, const uint32_t* __res
   const uint32_t flip = tab_eval<D>(tab + 32 * 3 * E, kk0, kk1, kk2, cnt) & a.valid;
   uint32_t pending = tab_eval<D>(tab + 33 * 3 * E, kk0, kk1, kk2, cnt) & a.valid;
   uint32_t lt = 0u;
-#pragma unroll 1
-  for (int qq = 0; qq < 8; ++qq) {
-    if (!pending) break;
-    const ojd::u4 r =
-        ojd::philox(site, sweep, grp, ((uint32_t)qq << 16) | ((uint32_t)q << 8) | ojd::TAG_SQA_SPLIT, a.keys);
+  auto draw = [&](int qq) {
+    return ojd::philox(site, sweep, grp, ((uint32_t)qq << 16) | ((uint32_t)q << 8) | ojd::TAG_SQA_SPLIT, a.keys);
+  };
+  auto levels = [&](int qq, const ojd::u4& r) {
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
       const uint32_t wl = ojd::pick(r, l);
@@ -208,13 +214,23 @@ __device__ __forceinline__ uint32_t split_site(uint32_t x, const uint32_t* __res
       lt |= pending & pm & ~wl;
       pending &= ~(pm ^ wl);
     }
+  };
+  if constexpr (DR > 1) {
+    if (!pending) return x ^ flip;
+    ojd::u4 r[DR];
+#pragma unroll
+    for (int qq = 0; qq < DR; ++qq) r[qq] = draw(qq);
+#pragma unroll
+    for (int qq = 0; qq < DR; ++qq) levels(qq, r[qq]);
   }
+#pragma unroll 1
+  for (int qq = DR > 1 ? DR : 0; qq < 8 && pending; ++qq) levels(qq, draw(qq));
   return x ^ flip ^ lt;
 }
 
 // Updates slots [lo, hi) of half X; returns the spins this thread flipped.
 // DOM: the sweep's live classes allow tab_eval_dominated.
-template <int D, bool DOM>
+template <int D, bool DOM, int DR>
 __device__ __forceinline__ uint32_t split_range(int lo, int hi, uint32_t* __restrict__ X,
                                                 const uint32_t* __restrict__ Y, const int32_t* __restrict__ gid,
                                                 const uint16_t* __restrict__ jm, const uint16_t* __restrict__ nbr,
@@ -226,11 +242,11 @@ __device__ __forceinline__ uint32_t split_range(int lo, int hi, uint32_t* __rest
     for (int s = lo + threadIdx.x; s < hi; s += 2 * T) {
       const int s2 = s + T;
       const uint32_t x0 = X[s];
-      const uint32_t v = split_site<D, DOM>(x0, X, nbr + (size_t)s * D, jm[s], Y[s], q, a, tab, (uint32_t)gid[s], k, g);
+      const uint32_t v = split_site<D, DOM, DR>(x0, X, nbr + (size_t)s * D, jm[s], Y[s], q, a, tab, (uint32_t)gid[s], k, g);
       if (s2 < hi) {
         const uint32_t x2 = X[s2];
         const uint32_t w2 =
-            split_site<D, DOM>(x2, X, nbr + (size_t)s2 * D, jm[s2], Y[s2], q, a, tab, (uint32_t)gid[s2], k, g);
+            split_site<D, DOM, DR>(x2, X, nbr + (size_t)s2 * D, jm[s2], Y[s2], q, a, tab, (uint32_t)gid[s2], k, g);
         X[s2] = w2;
         nf += __popc(w2 ^ x2);
       }
@@ -240,7 +256,7 @@ __device__ __forceinline__ uint32_t split_range(int lo, int hi, uint32_t* __rest
   } else {
     for (int s = lo + threadIdx.x; s < hi; s += T) {
       const uint32_t x0 = X[s];
-      const uint32_t v = split_site<D, DOM>(x0, X, nbr + (size_t)s * D, jm[s], Y[s], q, a, tab, (uint32_t)gid[s], k, g);
+      const uint32_t v = split_site<D, DOM, DR>(x0, X, nbr + (size_t)s * D, jm[s], Y[s], q, a, tab, (uint32_t)gid[s], k, g);
       X[s] = v;
       nf += __popc(v ^ x0);
     }
@@ -251,12 +267,14 @@ __device__ __forceinline__ uint32_t split_range(int lo, int hi, uint32_t* __rest
 // Shared memory: E[slots] | O[slots] | gid[nlocmax] | jm[nlocmax] | nbr[nlocmax][D]
 // CL: the group's sites are split over a cluster of CTAs (halo exchange);
 // without it one CTA owns all sites and a phase ends with one block barrier.
-template <int D, bool CL>
+template <int D, bool CL, int DR>
 __global__ void __launch_bounds__(kSplitMaxThreads) sqa_split_kernel(SplitArgs a) {
   extern __shared__ __align__(16) uint32_t sh[];
   constexpr int NC = (D + 1) * 3;
   constexpr int E = SplitTab<D>::E;
-  __shared__ __align__(16) uint32_t tab[SplitTab<D>::WORDS];
+  // CL: one sweep's tables; else this sweep's and the next one's
+  __shared__ __align__(16) uint32_t tabs[CL ? 1 : 2][SplitTab<D>::WORDS];
+  __shared__ uint32_t raw[NC + 2];  // CL: the sweep's thresholds, its always and live masks
   const int p = CL ? (int)cg::this_cluster().block_rank() : 0;
   const int g = blockIdx.y;
   const int32_t* gid_g = a.gidx + (size_t)p * a.slots;
@@ -291,33 +309,67 @@ __global__ void __launch_bounds__(kSplitMaxThreads) sqa_split_kernel(SplitArgs a
   unsigned long long nflip = 0;
   int prev_c = -1, prev_q = 0;  // colour class and half updated by the previous phase
   const uint32_t gg = a.group0 + (uint32_t)g;
-  for (int64_t k = 0; k < a.nsweeps; ++k) {
-    {
-      // the sweep's tables (every thread finished the previous sweep's last
-      // phase at its closing barrier)
-      const uint32_t alw = __ldg(a.mode + 2 * k), live = __ldg(a.mode + 2 * k + 1);
-      for (int idx = threadIdx.x; idx < SplitTab<D>::WORDS; idx += blockDim.x) {
-        const int row = idx / (3 * E), kq = (idx / E) % 3, u = idx % E;
-        uint32_t w = 0u;
-        if (u <= D) {
-          const int c = 3 * u + kq;
-          bool on;
-          if (row < 32)
-            on = ((live >> c) & 1u) && ((__ldg(a.thr + (size_t)k * NC + c) >> (31 - row)) & 1u);
-          else
-            on = row == 32 ? ((alw >> c) & 1u) : ((live >> c) & 1u);
-          w = on ? 0xFFFFFFFFu : 0u;
-        }
-        tab[idx] = w;
+  // table words of a sweep from its thresholds and masks
+  auto fill_tab = [&](uint32_t* tab, uint32_t alw, uint32_t live, auto thr_of) {
+    for (int idx = threadIdx.x; idx < SplitTab<D>::WORDS; idx += blockDim.x) {
+      const int row = idx / (3 * E), kq = (idx / E) % 3, u = idx % E;
+      uint32_t w = 0u;
+      if (u <= D) {
+        const int c = 3 * u + kq;
+        bool on;
+        if (row < 32)
+          on = ((live >> c) & 1u) && ((thr_of(c) >> (31 - row)) & 1u);
+        else
+          on = row == 32 ? ((alw >> c) & 1u) : ((live >> c) & 1u);
+        w = on ? 0xFFFFFFFFu : 0u;
       }
+      tab[idx] = w;
+    }
+  };
+  auto fill_from_global = [&](int64_t k) {
+    fill_tab(tabs[CL ? 0 : k & 1], __ldg(a.mode + 2 * k), __ldg(a.mode + 2 * k + 1),
+             [&](int c) { return __ldg(a.thr + (size_t)k * NC + c); });
+  };
+  // CL: the thresholds and masks of the next sweep are loaded during the current
+  // one, so that no load stands between a cluster's barriers
+  auto load_raw = [&](int64_t k) -> uint32_t {
+    const int t = threadIdx.x;
+    if (k >= a.nsweeps || t >= NC + 2) return 0u;
+    return t < NC ? __ldg(a.thr + (size_t)k * NC + t) : __ldg(a.mode + 2 * k + (t - NC));
+  };
+  uint32_t next = 0u, live_k = 0u, live_n = 0u;
+  if constexpr (CL) {
+    next = load_raw(0);
+  } else if (a.nsweeps > 0) {
+    live_n = __ldg(a.mode + 1);
+    fill_from_global(0);
+    __syncthreads();
+  }
+  for (int64_t k = 0; k < a.nsweeps; ++k) {
+    const uint32_t* tab = tabs[CL ? 0 : k & 1];
+    if constexpr (CL) {
+      // (every thread finished the previous sweep's last phase at its closing barrier)
+      if (threadIdx.x < NC + 2) raw[threadIdx.x] = next;
       __syncthreads();
+      next = load_raw(k + 1);
+      live_k = raw[NC + 1];
+      fill_tab(tabs[0], raw[NC], live_k, [&](int c) { return raw[c]; });
+      __syncthreads();
+    } else {
+      // the next sweep's tables, published by this sweep's closing barrier: the
+      // warps that are done with a phase wait for the loads while others work
+      live_k = live_n;
+      if (k + 1 < a.nsweeps) {
+        live_n = __ldg(a.mode + 2 * (k + 1) + 1);
+        fill_from_global(k + 1);
+      }
     }
     const uint32_t kk = a.sweep0 + (uint32_t)k;
     // the sweep's live classes allow the Trotter-dominated table evaluation
-    const bool dom = (__ldg(a.mode + 2 * k + 1) & split_not_dominated_mask<D>()) == 0u;
+    const bool dom = (live_k & split_not_dominated_mask<D>()) == 0u;
     auto range = [&](int lo, int hi, uint32_t* X, const uint32_t* Y, int q) {
-      return dom ? split_range<D, true>(lo, hi, X, Y, gid, jm, nbr, q, a, tab, kk, gg)
-                 : split_range<D, false>(lo, hi, X, Y, gid, jm, nbr, q, a, tab, kk, gg);
+      return dom ? split_range<D, true, DR>(lo, hi, X, Y, gid, jm, nbr, q, a, tab, kk, gg)
+                 : split_range<D, false, DR>(lo, hi, X, Y, gid, jm, nbr, q, a, tab, kk, gg);
     };
     for (int q = 0; q < 2; ++q) {
       uint32_t* X = q ? WO : WE;
@@ -401,27 +453,18 @@ size_t split_smem_bytes(const MscPlan& pl) {
   return (size_t)pl.slots * 8 + (size_t)pl.nlocmax * (4 + 2 + 2 * pl.D) + 16;
 }
 
-int split_threads() {
-  int threads = kSplitDefaultThreads;
-  if (const char* env = std::getenv("OJ_SQA_THREADS")) {
-    const int v = std::atoi(env);
-    if (v >= 32 && v <= kSplitMaxThreads && v % 32 == 0) threads = v;
-  }
-  return threads;
-}
-
 template <int D>
 cudaError_t launch_d(const MscPlan& pl, const SplitArgs& a, int G, cudaStream_t st, int threads) {
   const size_t smem = split_smem_bytes(pl);
   if (smem > kSplitSmemBytes) return cudaErrorInvalidValue;
   if (pl.P == 1) {
-    auto k1 = sqa_split_kernel<D, false>;
+    auto k1 = sqa_split_kernel<D, false, kSplitDraws>;
     cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     k1<<<dim3(1, G, 1), threads, smem, st>>>(a);
     return cudaGetLastError();
   }
-  auto kern = sqa_split_kernel<D, true>;
+  auto kern = sqa_split_kernel<D, true, 1>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   if (pl.P > 8) {
@@ -445,7 +488,17 @@ cudaError_t launch_d(const MscPlan& pl, const SplitArgs& a, int G, cudaStream_t 
 
 }  // namespace
 
-int split_default_threads() { return split_threads(); }
+// Threads of a CTA: a whole group in one CTA takes one per site of its largest
+// class, but at least 256, which also write the tables (70 sites: 64 threads 5.6 us a
+// sweep, 256 5.1).
+int split_default_threads(const oj_graph* g, int P) {
+  if (const char* env = std::getenv("OJ_SQA_THREADS")) {
+    const int v = std::atoi(env);
+    if (v >= 32 && v <= kSplitMaxThreads && v % 32 == 0) return v;
+  }
+  if (P > 1) return kSplitDefaultThreads;
+  return std::max(256, std::min(kSplitDefaultThreads, (largest_class(g) + 31) / 32 * 32));
+}
 
 int sqa_split_replicas_per_group(int T) {
   const int H = T / 2;
@@ -459,12 +512,18 @@ bool sqa_split_applies(const oj_graph* g, int T) {
          T <= 64 && T % 2 == 0;
 }
 
-// Cluster size for G replica groups: as many CTAs per group as the SMs allow
-// (one CTA per SM), at least 256 sites per CTA, and a partition whose two
-// halves, halo and tables fit the shared-memory budget.
+// Cluster size for G replica groups: one CTA per group, or as many as all run at
+// once (at least 256 sites per CTA) where that is shorter, and a partition whose two
+// halves, halo and tables fit the shared-memory budget.  Time of a phase in us, from
+// 3-regular graphs: one CTA 0.45 + 0.0023 per site of the class; a cluster 2.3 for its
+// barrier and halo (2.8 below 16 CTAs) + 0.0023 per site of a CTA's class (us a sweep, one
+// CTA / a cluster: 1000 sites, T = 4 9.4 / 23.2; 4096 sites, T = 16, 8 replicas 22.2 / 16.1,
+// 64 replicas 22.2 / 23.1).
 cudaError_t sqa_split_prepare(oj_graph* g, int G, int sm_count, std::string* why, int cluster) {
-  int P = std::max(1, std::min(kSplitMaxCluster, sm_count / std::max(G, 1)));
+  int P = std::max(1, std::min(cluster_most(G), sm_count / std::max(G, 1)));
   while (P > 1 && g->n / P < 256) --P;
+  const double c = largest_class(g);
+  if (0.45 + 0.0023 * c <= (P == kSplitMaxCluster ? 2.3 : 2.8) + 0.0023 * c / P) P = 1;
   if (const char* env = std::getenv("OJ_SQA_CLUSTER")) {
     const int v = std::atoi(env);
     if (v >= 1 && v <= kSplitMaxCluster && v <= g->n) P = v;
@@ -483,7 +542,7 @@ cudaError_t sqa_split_prepare(oj_graph* g, int G, int sm_count, std::string* why
 cudaError_t launch_sqa_split(const oj_graph* g, int G, int T, uint32_t* words, const uint32_t* thr,
                              const uint32_t* mode, int64_t nsweeps, RngBase rb, cudaStream_t st, int* launches,
                              int threads) {
-  if (threads == 0) threads = split_threads();
+  if (threads == 0) threads = split_default_threads(g, g->msc->P);
   if (threads < 32 || threads > kSplitMaxThreads || threads % 32) return cudaErrorInvalidValue;
   const MscPlan& pl = *g->msc;
   SplitArgs a;

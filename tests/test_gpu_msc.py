@@ -48,3 +48,25 @@ def _circulant(n, d):
         pairs |= {(i, i + n // 2) for i in range(n // 2)}
     a, b = np.array(sorted(pairs)).T
     return I.augmented_from_ising(np.zeros(n), (a, b, rng.choice([-1.0, 1.0], size=a.size)), n), 0.0
+
+
+@pytest.mark.parametrize("which", [(40, 1), (70, 2), (130, 3), (1000, 3), (4200, 3), (300, 4), (200, 5), (96, 6),
+                                   (98, 7), (120, 8)])
+@pytest.mark.parametrize("T,R", [(2, 40), (8, 5), (32, 3), (64, 2)])
+def test_slice_split_forms_bit_exact(ctx, which, T, R):
+    """The slice-split SQA kernel's default shapes: one CTA per group and clusters,
+    tables written a sweep ahead or at the sweep's start, every degree."""
+    n, d = which
+    m, _ = I.random_regular_pm_j(n, d, seed=9, max_tries=10**5) if d < 4 else _circulant(n, d)
+    g = O.AugCSR(m)
+    dg = N.Graph(ctx, g.n, g.indptr, g.indices, g.data)
+    info = dg.info()
+    ss = np.array([0.0, 0.2, 0.6, 0.9, 1.0])
+    betas, mcs = np.full(5, 4.0), np.ones(5, np.int32)
+    s0 = np.random.default_rng(n + T).choice(np.array([-1, 1], np.int8), size=(R, T, n))
+    s = s0.copy()
+    st = N.sqa_run(dg, s, 1.0, betas, ss, mcs, seed=52, kernel="bitpacked")
+    a, b = O.sqa_coefficients(betas, ss, 1.0, T)
+    thr, mode = O.sqa_msc_thresholds(a, b, info["coupling_abs"], info["max_degree"])
+    np.testing.assert_array_equal(s, O.replay_sqa_split(g, s0, thr, mode, 52))
+    assert (st["cluster"] > 1) == (n == 4200 and R <= 8 * max(1, 32 // (T // 2)))
