@@ -361,7 +361,9 @@ __global__ void __launch_bounds__(W * 32, MINB) sa_batch_kernel(BatchArgs a) {
 // The exact fields of this lane's four sites (4 lane .. 4 lane + 3) of a
 // one-chunk instance: f_j = fp32(fp64(h_j) + 2^e sum_i q_ji s_i), the sum in
 // int64 (exact), the same operations as the tensor-core field kernel's
-// epilogue, so the same values.  wd: this lane's spin bits (set: -1).
+// epilogue, so the same values.  wd: this lane's spin bits (set: -1).  QS: Qm is in
+// shared memory.
+template <bool QS>
 __device__ __forceinline__ float4 exact_fields1(const int32_t* __restrict__ Qm, int n, uint32_t wd, double scale,
                                                 const float4 h4) {
   const int lane = threadIdx.x & 31;
@@ -373,7 +375,8 @@ __device__ __forceinline__ float4 exact_fields1(const int32_t* __restrict__ Qm, 
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
       const int i = 4 * L0 + t;
-      q[t] = i < n ? __ldg(reinterpret_cast<const int4*>(Qm + (size_t)i * 128) + lane) : make_int4(0, 0, 0, 0);
+      const int4* at = reinterpret_cast<const int4*>(Qm + (size_t)i * 128) + lane;
+      q[t] = i < n ? (QS ? *at : __ldg(at)) : make_int4(0, 0, 0, 0);
     }
     int p[4] = {0, 0, 0, 0};
 #pragma unroll
@@ -411,9 +414,12 @@ __device__ __forceinline__ float field_gap(const float4 f, const float4 g, int n
   return d;
 }
 
-template <int W, bool H>
+// QS: the grid integers Q of the recompute are staged in shared memory beside the
+// couplings (a recompute's 13 passes over 100 rows then wait for no L2 round trip;
+// 100 sites, 100 reads, 1000 sweeps 1.94 -> 1.79 ms).
+template <int W, bool H, bool QS>
 __global__ void __launch_bounds__(W * 32) sa_batch1_kernel(BatchArgs a) {
-  extern __shared__ __align__(16) float shb[];  // [n][128] couplings of the item's instance
+  extern __shared__ __align__(16) float shb[];  // [n][128] couplings of the item's instance, then Q (QS)
   __shared__ int item_sh;
   __shared__ __align__(8) uint64_t stage_bar;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -437,6 +443,8 @@ __global__ void __launch_bounds__(W * 32) sa_batch1_kernel(BatchArgs a) {
       const void* src = H ? static_cast<const void*>(a.J16 + a.joff[m]) : static_cast<const void*>(a.J + a.joff[m]);
       if (!stage_rows(shb, src, (uint32_t)(n * 128 * (H ? 2 : 4)), &stage_bar, stage_phase, a)) continue;
     }
+    char* qsh = reinterpret_cast<char*>(shb) + (size_t)n * 128 * (H ? 2 : 4);
+    if (QS && !stage_rows(qsh, a.Q + a.joff[m], (uint32_t)(n * 128 * 4), &stage_bar, stage_phase, a)) continue;
     if (r >= a.reads[m]) continue;  // warps past the instance's reads wait for the next item
     int8_t* gs = a.spins + a.soff[m] + (size_t)r * n;
     uint32_t wd = 0u;  // bit e: site 4*lane + e is -1
@@ -451,14 +459,14 @@ __global__ void __launch_bounds__(W * 32) sa_batch1_kernel(BatchArgs a) {
     const __half* Js16 = reinterpret_cast<const __half*>(shb) + 4 * lane;
     const uint32_t tag = ((a.inst0 + (uint32_t)m) << 8) | ojd::TAG_BATCH;
     const uint32_t rg = a.rep0 + (uint32_t)r;
-    const int32_t* Qm = a.Q ? a.Q + a.joff[m] : nullptr;
+    const int32_t* Qm = QS ? reinterpret_cast<const int32_t*>(qsh) : (a.Q ? a.Q + a.joff[m] : nullptr);
     const double qscale = Qm ? ldexp(1.0, a.uexp[m]) : 0.0;
     const float4 h4q = Qm ? ldg4(a.h + a.hoff[m] + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
     float dmax = 0.0f;
     for (int64_t k = 0; k < a.nsweeps; ++k) {
       const float beta2 = 2.0f * __ldg(a.betas + k);
       if (Qm && k > 0 && (a.sweep0 + (uint32_t)k) % (uint32_t)a.recompute == 0u) {
-        const float4 fx = exact_fields1(Qm, n, wd, qscale, h4q);
+        const float4 fx = exact_fields1<QS>(Qm, n, wd, qscale, h4q);
         if (a.drift) dmax = fmaxf(dmax, field_gap(fc, fx, n));
         fc = fx;
       }
@@ -509,7 +517,7 @@ __global__ void __launch_bounds__(W * 32) sa_batch1_kernel(BatchArgs a) {
     }
     if (Qm && a.drift) {
       // the drift check after the last sweep; the exact fields are kept
-      const float4 fx = exact_fields1(Qm, n, wd, qscale, h4q);
+      const float4 fx = exact_fields1<QS>(Qm, n, wd, qscale, h4q);
       dmax = fmaxf(dmax, field_gap(fc, fx, n));
       fc = fx;
 #pragma unroll
@@ -658,12 +666,15 @@ int batch_variant_max_n(int variant) {
 // group of loads, and more warps hide it.  Larger instances take 45, which has
 // eight chunks' loads in flight: 2048 sites, 4096 replicas, 1000 sweeps 21.9
 // (83), 22.3 (82), 20.0 ms (45); 520 to 2048 sites with 8 to 4096 replicas 2 to 24 %
-// less; 64 instances of 64 to 512 sites with 32 reads 6.4 (83), 7.1 ms (45).
-int batch_default_variant(int max_n) {
+// less; 64 instances of 64 to 512 sites with 32 reads 6.4 (83), 7.1 ms (45).  One-chunk
+// batches with at most eight replicas an SM spread them over more CTAs of four warps
+// (100 sites, 100 reads, 1000 sweeps 2.17 (83), 1.94 ms (45)).
+int batch_default_variant(int max_n, int64_t replicas, int sm_count) {
   if (const char* env = std::getenv("OJ_BATCH_VARIANT")) {
     const int v = std::atoi(env);
     if (batch_variant_valid(v)) return v;
   }
+  if (max_n <= 128) return replicas <= 8 * (int64_t)sm_count ? 45 : 83;
   return max_n > 512 ? 45 : 83;
 }
 
@@ -687,8 +698,11 @@ cudaError_t launch_variant(const BatchArgs& a, int nitems, int sm_count, cudaStr
 
 template <int W>
 cudaError_t launch_one_chunk(const BatchArgs& a, int max_n, int nitems, int sm_count, cudaStream_t st, bool h) {
-  auto kern = h ? sa_batch1_kernel<W, true> : sa_batch1_kernel<W, false>;
-  const size_t smem = (size_t)max_n * 128 * (h ? 2 : 4);  // the staged couplings
+  // Q beside the couplings where every CTA has an SM to itself anyway
+  const bool qs = a.Q && nitems <= sm_count;
+  auto kern = h ? (qs ? sa_batch1_kernel<W, true, true> : sa_batch1_kernel<W, true, false>)
+                : (qs ? sa_batch1_kernel<W, false, true> : sa_batch1_kernel<W, false, false>);
+  const size_t smem = (size_t)max_n * 128 * ((h ? 2 : 4) + (qs ? 4 : 0));
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
@@ -707,7 +721,6 @@ cudaError_t launch_batch_sweeps(const oj_batch* b, const int32_t* d_reads, const
                                 const int64_t* d_foff, double* d_energies, const int64_t* d_eoff,
                                 bool write_fields, int* d_status, long long wait_limit,
                                 const int32_t* kstart, int recompute, unsigned int* d_drift) {
-  if (variant == 0) variant = batch_default_variant(b->max_n);
   if (!batch_variant_valid(variant) || b->max_n > batch_variant_max_n(variant)) return cudaErrorInvalidValue;
   if (b->count == 0 || nitems <= 0 || nsweeps <= 0) return cudaSuccess;
   const int fstride = std::max(128, (b->max_n + 127) / 128 * 128);
