@@ -509,10 +509,7 @@ __global__ void unpack_kernel(const uint32_t* __restrict__ words, int R, int n, 
 
 int sa_colour_max_smem_sites() { return kSmemBudget; }
 
-// Builds the graph's ColourPlan (once).
-cudaError_t colour_prepare(oj_graph* g) {
-  const std::lock_guard<std::mutex> lock(g->cplan_lock);
-  if (g->cplan) return cudaSuccess;
+static cudaError_t colour_build(oj_graph* g) {
   const int n = g->n, ncol = g->info.num_colours;
   std::vector<int32_t> order(g->order), slot(n);
   std::vector<int4> cls(ncol);
@@ -576,6 +573,19 @@ cudaError_t colour_prepare(oj_graph* g) {
   }
   g->cplan = std::move(plan);
   return cudaSuccess;
+}
+
+// Builds the graph's ColourPlan (once).  No exception leaves it: its callers
+// are reached through the C interface, and a host allocation that fails is
+// reported as out of memory.
+cudaError_t colour_prepare(oj_graph* g) {
+  const std::lock_guard<std::mutex> lock(g->cplan_lock);
+  if (g->cplan) return cudaSuccess;
+  try {
+    return colour_build(g);
+  } catch (...) {
+    return cudaErrorMemoryAllocation;
+  }
 }
 
 namespace {

@@ -323,9 +323,8 @@ int sw_threads(const oj_graph* g, int R, int sm_count) {
 }
 
 // Bond list of the graph: (i, j) with i < j from the neighbour lists, then
-// (i, n) for every non-zero h_i; built once per graph.
-cudaError_t sw_prepare(oj_graph* g) {
-  if (g->sw_ne >= 0) return cudaSuccess;
+// (i, n) for every non-zero h_i.
+static cudaError_t sw_build(oj_graph* g) {
   std::vector<int32_t> ei, ej;
   std::vector<float> w;
   std::vector<uint8_t> pos;
@@ -370,6 +369,17 @@ cudaError_t sw_prepare(oj_graph* g) {
   }
   g->sw_ne = (int64_t)ne;
   return cudaSuccess;
+}
+
+// Builds the bond list once per graph; a host allocation that fails is
+// reported as out of memory, no exception reaches the C interface.
+cudaError_t sw_prepare(oj_graph* g) {
+  if (g->sw_ne >= 0) return cudaSuccess;
+  try {
+    return sw_build(g);
+  } catch (...) {
+    return cudaErrorMemoryAllocation;
+  }
 }
 
 cudaError_t launch_sw(const oj_graph* g, int R, int8_t* spins, const float* betas, int64_t nsweeps, RngBase rb,
