@@ -165,6 +165,13 @@ __device__ __forceinline__ float neglog_gap(float x, uint32_t word) {
 // memory, no multicast).  Every wait is bounded by an iteration count.
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// Kernels launched early (launch_early): grid_wait returns when every kernel
+// before this one on the stream has completed and its writes can be seen (at
+// once for an ordinary launch); after grid_release by all its CTAs the next
+// early kernel may start up to its own grid_wait.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count));
 }

@@ -291,6 +291,24 @@ cudaError_t launch_hot_tc(const oj_batch* b, const int32_t* d_reads, const int64
                           float* F, const int64_t* d_foff, const int64_t* d_eoff, const int32_t* d_items,
                           int nitems, const float* betas, int64_t nsweeps, RngBase rb, uint32_t inst0,
                           int32_t* kstop, int* d_status, long long wait_limit, cudaStream_t st);
+// Launches a kernel of one argument; early, its CTAs may start before the
+// kernel before it on the stream has completed (that one must be a kernel, with
+// no copy between), up to their ojd::grid_wait.
+template <class Args>
+cudaError_t launch_early(void (*kern)(Args), int grid, int block, size_t smem, cudaStream_t st, bool early,
+                         const Args& a) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, a);
+}
 // Fields on the tensor cores, then the sweeps (one segment, no recompute).
 cudaError_t launch_sa_batch(const oj_batch* b, const int32_t* d_reads, const int64_t* d_soff,
                             const int32_t* d_items, int nitems, int* d_counter, int8_t* spins, const float* betas,
@@ -302,18 +320,21 @@ void field_tc_items(const oj_batch* b, const int32_t* reads, const std::vector<i
                     std::vector<int32_t>& items);
 cudaError_t launch_field_tc(const oj_batch* b, const int32_t* d_reads, const int64_t* d_soff, const int8_t* spins,
                             float* F, const int64_t* d_foff, const int32_t* d_items, int nitems, int NT, bool compare,
-                            unsigned int* d_drift, int* d_status, long long wait_limit, cudaStream_t st);
+                            unsigned int* d_drift, int* d_status, long long wait_limit, cudaStream_t st,
+                            int* d_counter = nullptr, bool early = false);
 cudaError_t field_tc_prepare(oj_batch* b, const std::vector<float>& J32, const std::vector<int64_t>& joff,
                              const std::vector<int8_t>* J8, int pmax);
 // The batched sweep kernel alone (no fields): nsweeps sweeps from the fields in
-// d_fields; with write_fields it stores its final fields back there.
+// d_fields; with write_fields it stores its final fields back there.  early:
+// right after launch_field_tc with this call's counter, which has set it to zero.
 cudaError_t launch_batch_sweeps(const oj_batch* b, const int32_t* d_reads, const int64_t* d_soff,
                                 const int32_t* d_items, int nitems, int* d_counter, int8_t* spins,
                                 const float* betas, int64_t nsweeps, RngBase rb, uint32_t inst0, int sm_count,
                                 cudaStream_t st, int* launches, int variant, float* d_fields,
                                 const int64_t* d_foff, double* d_energies, const int64_t* d_eoff,
                                 bool write_fields, int* d_status, long long wait_limit,
-                                const int32_t* kstart = nullptr, int recompute = 0, unsigned int* d_drift = nullptr);
+                                const int32_t* kstart = nullptr, int recompute = 0, unsigned int* d_drift = nullptr,
+                                bool early = false);
 cudaError_t launch_batch_energy(const oj_batch* b, const int32_t* d_reads, const int64_t* d_soff,
                                 const int64_t* d_eoff, const int32_t* d_order, int max_reads, const int8_t* spins,
                                 double* out, cudaStream_t st, int nsplit, double* parts, int64_t nrep);

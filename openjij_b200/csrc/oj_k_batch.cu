@@ -182,6 +182,9 @@ __global__ void __launch_bounds__(W * 32, MINB) sa_batch_kernel(BatchArgs a) {
   uint32_t stage_phase = 0u;
   if (SJ) stage_init(&stage_bar);
   unsigned long long nflip = 0;  // lane 0 counts the warp's flips
+  // the field kernel before has finished; the one after may set itself up
+  ojd::grid_wait();
+  ojd::grid_release();
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) item_sh = atomicAdd(a.counter, 1);
@@ -221,8 +224,10 @@ __global__ void __launch_bounds__(W * 32, MINB) sa_batch_kernel(BatchArgs a) {
     __syncwarp();
     // the fields f_j = h_j + sum_i J_ij s_i come from the tensor-core field kernel
     {
+      // written while this kernel may already have been launched: not by __ldg
       const float* Fr = a.F + a.foff[m] + (size_t)r * npad;
-      for (int c = 0; c < nch; ++c) reinterpret_cast<float4*>(f)[32 * c + lane] = ldg4(Fr + 128 * c + 4 * lane);
+      for (int c = 0; c < nch; ++c)
+        reinterpret_cast<float4*>(f)[32 * c + lane] = __ldcg(reinterpret_cast<const float4*>(Fr + 128 * c) + lane);
     }
     __syncwarp();
     const uint32_t tag = ((a.inst0 + (uint32_t)m) << 8) | ojd::TAG_BATCH;
@@ -679,7 +684,8 @@ int batch_default_variant(int max_n, int64_t replicas, int sm_count) {
 }
 
 template <int W, int MINB, int GROUP>
-cudaError_t launch_variant(const BatchArgs& a, int nitems, int sm_count, cudaStream_t st, bool h, size_t jbytes) {
+cudaError_t launch_variant(const BatchArgs& a, int nitems, int sm_count, cudaStream_t st, bool h, size_t jbytes,
+                           bool early) {
   const bool sj = jbytes > 0;
   auto kern = h ? (sj ? sa_batch_kernel<W, MINB, GROUP, true, true> : sa_batch_kernel<W, MINB, GROUP, true, false>)
                 : (sj ? sa_batch_kernel<W, MINB, GROUP, false, true> : sa_batch_kernel<W, MINB, GROUP, false, false>);
@@ -692,8 +698,7 @@ cudaError_t launch_variant(const BatchArgs& a, int nitems, int sm_count, cudaStr
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
   const int grid = std::max(1, std::min(nitems, per_sm * sm_count));
-  kern<<<grid, W * 32, smem, st>>>(a);
-  return cudaGetLastError();
+  return launch_early(kern, grid, W * 32, smem, st, early, a);
 }
 
 template <int W>
@@ -720,7 +725,7 @@ cudaError_t launch_batch_sweeps(const oj_batch* b, const int32_t* d_reads, const
                                 cudaStream_t st, int* launches, int variant, float* d_fields,
                                 const int64_t* d_foff, double* d_energies, const int64_t* d_eoff,
                                 bool write_fields, int* d_status, long long wait_limit,
-                                const int32_t* kstart, int recompute, unsigned int* d_drift) {
+                                const int32_t* kstart, int recompute, unsigned int* d_drift, bool early) {
   if (!batch_variant_valid(variant) || b->max_n > batch_variant_max_n(variant)) return cudaErrorInvalidValue;
   if (b->count == 0 || nitems <= 0 || nsweeps <= 0) return cudaSuccess;
   const int fstride = std::max(128, (b->max_n + 127) / 128 * 128);
@@ -760,7 +765,7 @@ cudaError_t launch_batch_sweeps(const oj_batch* b, const int32_t* d_reads, const
   a.uexp = own ? b->d_uexp.as<int32_t>() : nullptr;
   a.recompute = own ? recompute : 0;
   a.drift = own ? d_drift : nullptr;
-  cudaError_t e = cudaMemsetAsync(d_counter, 0, sizeof(int), st);
+  cudaError_t e = early ? cudaSuccess : cudaMemsetAsync(d_counter, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
   if (b->max_n <= 128) {
     // one chunk per instance: fields and spin bits in registers (same warps
@@ -778,12 +783,12 @@ cudaError_t launch_batch_sweeps(const oj_batch* b, const int32_t* d_reads, const
   size_t jbytes = (size_t)b->max_n * (size_t)fstride * (b->j16 ? 2 : 4);
   if (jbytes > kBatchSmemJBytes) jbytes = 0;
   switch (variant) {
-    case 45: e = launch_variant<4, 5, 8>(a, nitems, sm_count, st, b->j16, jbytes); break;
-    case 82: e = launch_variant<8, 2, 16>(a, nitems, sm_count, st, b->j16, jbytes); break;
-    case 83: e = launch_variant<8, 3, 4>(a, nitems, sm_count, st, b->j16, jbytes); break;
-    case 84: e = launch_variant<8, 4, 4>(a, nitems, sm_count, st, b->j16, jbytes); break;
-    case 162: e = launch_variant<16, 2, 4>(a, nitems, sm_count, st, b->j16, jbytes); break;
-    default: e = launch_variant<32, 1, 4>(a, nitems, sm_count, st, b->j16, jbytes); break;
+    case 45: e = launch_variant<4, 5, 8>(a, nitems, sm_count, st, b->j16, jbytes, early); break;
+    case 82: e = launch_variant<8, 2, 16>(a, nitems, sm_count, st, b->j16, jbytes, early); break;
+    case 83: e = launch_variant<8, 3, 4>(a, nitems, sm_count, st, b->j16, jbytes, early); break;
+    case 84: e = launch_variant<8, 4, 4>(a, nitems, sm_count, st, b->j16, jbytes, early); break;
+    case 162: e = launch_variant<16, 2, 4>(a, nitems, sm_count, st, b->j16, jbytes, early); break;
+    default: e = launch_variant<32, 1, 4>(a, nitems, sm_count, st, b->j16, jbytes, early); break;
   }
   if (e == cudaSuccess && launches) ++*launches;
   return e;

@@ -67,6 +67,7 @@ struct FieldArgs {
   unsigned int* drift;     // float bits (non-negative values order as integers)
   int* status;
   long long wait_limit;    // iterations of a pipeline wait (0: give up at once)
+  int* counter;            // the next sweep kernel's item counter, set to zero here (or null)
 };
 
 using ojd::bulk_copy;
@@ -247,6 +248,13 @@ __global__ void __launch_bounds__(kFieldThreads, 1) field_tc_kernel(FieldArgs a)
   };
   if (tid == 0)
     for (int u = 0; u < ST - 1 && u < nu; ++u) issue_a(u);
+  // so far only what no launch writes (tables, digits); the spins, F, the drift
+  // and the counter are the sweep kernel's before this one.  No grid_release
+  // here: sweep CTAs that come in while this kernel's CTAs leave pile up on some
+  // SMs (64 instances of 64 to 512 sites 7.60 ms with one before the epilogue,
+  // 6.25 without; 777 sites 5.56 and 5.53)
+  ojd::grid_wait();
+  if (a.counter && item == 0 && tid == 0) *a.counter = 0;
   for (int u = 0; u < ST - 1; ++u) {
     if (u < nu) issue_b(u);
     else cp_async_commit();  // an empty group keeps the count per chunk
@@ -365,7 +373,7 @@ __global__ void __launch_bounds__(kFieldThreads, 1) field_tc_kernel(FieldArgs a)
 }
 
 template <int D, int NT>
-cudaError_t launch_field_dn(const FieldArgs& a, cudaStream_t st) {
+cudaError_t launch_field_dn(const FieldArgs& a, cudaStream_t st, bool early) {
   using S = FieldShape<D, NT>;
   auto kern = field_tc_kernel<D, NT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem);
@@ -375,19 +383,18 @@ cudaError_t launch_field_dn(const FieldArgs& a, cudaStream_t st) {
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFieldThreads, S::kSmem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1 || (size_t)per_sm * S::kCols > 512) return cudaErrorInvalidConfiguration;
-  kern<<<a.nitems, kFieldThreads, S::kSmem, st>>>(a);
-  return cudaGetLastError();
+  return launch_early(kern, a.nitems, kFieldThreads, S::kSmem, st, early, a);
 }
 
 template <int D>
-cudaError_t launch_field_d(const FieldArgs& a, int NT, cudaStream_t st) {
+cudaError_t launch_field_d(const FieldArgs& a, int NT, cudaStream_t st, bool early) {
   switch (NT) {
-    case 16: return launch_field_dn<D, 16>(a, st);
-    case 32: return launch_field_dn<D, 32>(a, st);
-    case 64: return launch_field_dn<D, 64>(a, st);
-    case 128: return launch_field_dn<D, 128>(a, st);
+    case 16: return launch_field_dn<D, 16>(a, st, early);
+    case 32: return launch_field_dn<D, 32>(a, st, early);
+    case 64: return launch_field_dn<D, 64>(a, st, early);
+    case 128: return launch_field_dn<D, 128>(a, st, early);
     default:
-      if constexpr (D == 1) return launch_field_dn<1, 256>(a, st);
+      if constexpr (D == 1) return launch_field_dn<1, 256>(a, st, early);
       return cudaErrorInvalidValue;
   }
 }
@@ -430,7 +437,8 @@ void field_tc_items(const oj_batch* b, const int32_t* reads, const std::vector<i
 
 cudaError_t launch_field_tc(const oj_batch* b, const int32_t* d_reads, const int64_t* d_soff, const int8_t* spins,
                             float* F, const int64_t* d_foff, const int32_t* d_items, int nitems, int NT, bool compare,
-                            unsigned int* d_drift, int* d_status, long long wait_limit, cudaStream_t st) {
+                            unsigned int* d_drift, int* d_status, long long wait_limit, cudaStream_t st, int* d_counter,
+                            bool early) {
   if (nitems <= 0) return cudaSuccess;
   FieldArgs a;
   a.digits = b->d_dig.as<int8_t>();
@@ -450,7 +458,8 @@ cudaError_t launch_field_tc(const oj_batch* b, const int32_t* d_reads, const int
   a.drift = d_drift;
   a.status = d_status;
   a.wait_limit = wait_limit >= 0 ? wait_limit : kDrainLimit;
-  return b->ndig == 1 ? launch_field_d<1>(a, NT, st) : launch_field_d<4>(a, NT, st);
+  a.counter = d_counter;
+  return b->ndig == 1 ? launch_field_d<1>(a, NT, st, early) : launch_field_d<4>(a, NT, st, early);
 }
 
 // Host side: the grid of every instance and its digits, tiled.  Instance m's
