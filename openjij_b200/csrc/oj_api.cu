@@ -855,11 +855,14 @@ oj_status oj_sa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int8_t* spins, c
     FieldCall fc;
     if (oj_status fs = field_call(ctx, g->single.get(), &hreads, std::vector<int>{0}, R, &fc)) return fs;
     if (tit == g->tuned.end() && autotune_requested(flags) && S > 0) {
-      // candidates run 16 sweeps with betas spread over the schedule on a copy of the spins
+      // Candidates run up to 128 sweeps with betas spread over the schedule on a copy
+      // of the spins: the start's many flips weigh less there than in 32 sweeps, which
+      // chose variant 82 for 2048 sites and 4096 replicas (22.3 ms a 1000-sweep call;
+      // variant 45, chosen with 128, 21.1).
       std::vector<int> cand;
       for (int v : {45, 82, 83, 84, 162, 321})
         if (n <= batch_variant_max_n(v)) cand.push_back(v);
-      const int64_t Ssub = std::min<int64_t>(S, 32);
+      const int64_t Ssub = std::min<int64_t>(S, 128);
       std::vector<float> tb(Ssub);
       for (int64_t q = 0; q < Ssub; ++q) tb[q] = bf[(size_t)((q * S) / Ssub)];
       const size_t sb_al = al(spin_bytes);
