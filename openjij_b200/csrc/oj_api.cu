@@ -1505,7 +1505,7 @@ oj_status build_batch(oj_ctx* ctx, int32_t count, const int32_t* n, const int64_
   auto up = [&](DevBuf& d, const void* src, size_t bytes) -> cudaError_t {
     cudaError_t e = d.ensure(std::max<size_t>(bytes, 16));
     if (e != cudaSuccess) return e;
-    return bytes ? cudaMemcpy(d.ptr, src, bytes, cudaMemcpyHostToDevice) : cudaSuccess;
+    return bytes ? copy_tables(d.ptr, src, bytes) : cudaSuccess;
   };
   OJ_CK(up(b->d_J, J32.data(), J32.size() * 4), "upload J");
   // flip rows in half the bytes when FP16 holds every FP32 coupling exactly

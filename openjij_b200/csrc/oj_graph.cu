@@ -155,7 +155,7 @@ static cudaError_t upload(DevBuf& b, const std::vector<T>& v) {
   const size_t bytes = std::max<size_t>(v.size() * sizeof(T), 16);
   cudaError_t e = b.ensure(bytes);
   if (e != cudaSuccess || v.empty()) return e;
-  return cudaMemcpy(b.ptr, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+  return copy_tables(b.ptr, v.data(), v.size() * sizeof(T));
 }
 
 // Builds everything from the augmented CSR (rows sorted or not).

@@ -50,6 +50,16 @@ struct DevBuf {
   }
 };
 
+// Tables from pageable host memory to the device, there when it returns.
+// cudaMemcpy alone may return as soon as it has staged the data, and a context's
+// stream, created non-blocking, does not wait for the legacy stream that the copy
+// is on: a launch right after it, or by another context that finds the tables
+// published, could read what was there before.
+inline cudaError_t copy_tables(void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(cudaStreamLegacy);
+}
+
 // Partition of the sites of a regular +-c graph over the CTAs of one thread
 // block cluster, used by the bit-packed SA kernel.  Each CTA (part p) keeps the
 // words of its own sites and a halo copy of remote neighbours in shared memory.

@@ -567,7 +567,7 @@ static cudaError_t colour_build(oj_graph* g) {
   std::memcpy(host.data() + b_site, cls.data(), cls.size() * 16);
   std::memcpy(host.data() + b_site + b_cls, slice.data(), slice.size() * 8);
   std::memcpy(host.data() + b_site + b_cls + b_slice, ent.data(), ent.size() * 8);
-  if ((e = cudaMemcpy(base, host.data(), host.size(), cudaMemcpyHostToDevice)) != cudaSuccess) {
+  if ((e = copy_tables(base, host.data(), host.size())) != cudaSuccess) {
     plan->tables.release();
     return e;
   }

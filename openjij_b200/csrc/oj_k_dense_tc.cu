@@ -528,7 +528,7 @@ cudaError_t dense_tc_prepare(oj_graph* g, std::string* why) {
   auto up = [&](DevBuf& b, const void* src, size_t bytes) -> cudaError_t {
     cudaError_t r = b.ensure(std::max<size_t>(bytes, 16));
     if (r != cudaSuccess || bytes == 0) return r;
-    return cudaMemcpy(b.ptr, src, bytes, cudaMemcpyHostToDevice);
+    return copy_tables(b.ptr, src, bytes);
   };
   if ((e = up(plan->bt_hi, hi.data(), hi.size() * 2)) != cudaSuccess) return e;
   if (!exact && (e = up(plan->bt_lo, lo.data(), lo.size() * 2)) != cudaSuccess) return e;

@@ -521,15 +521,15 @@ cudaError_t field_tc_prepare(oj_batch* b, const std::vector<float>& J32, const s
   cudaError_t err;
   if (q32) {
     if ((err = b->d_q32.ensure(Q.size() * 4)) != cudaSuccess) return err;
-    if ((err = cudaMemcpy(b->d_q32.ptr, Q.data(), Q.size() * 4, cudaMemcpyHostToDevice)) != cudaSuccess) return err;
+    if ((err = copy_tables(b->d_q32.ptr, Q.data(), Q.size() * 4)) != cudaSuccess) return err;
   }
   if ((err = b->d_dig.ensure(tiles.size())) != cudaSuccess) return err;
-  if ((err = cudaMemcpy(b->d_dig.ptr, tiles.data(), tiles.size(), cudaMemcpyHostToDevice)) != cudaSuccess) return err;
+  if ((err = copy_tables(b->d_dig.ptr, tiles.data(), tiles.size())) != cudaSuccess) return err;
   if ((err = b->d_dtoff.ensure(dtoff.size() * 8)) != cudaSuccess) return err;
-  if ((err = cudaMemcpy(b->d_dtoff.ptr, dtoff.data(), dtoff.size() * 8, cudaMemcpyHostToDevice)) != cudaSuccess)
+  if ((err = copy_tables(b->d_dtoff.ptr, dtoff.data(), dtoff.size() * 8)) != cudaSuccess)
     return err;
   if ((err = b->d_uexp.ensure(uexp.size() * 4)) != cudaSuccess) return err;
-  return cudaMemcpy(b->d_uexp.ptr, uexp.data(), uexp.size() * 4, cudaMemcpyHostToDevice);
+  return copy_tables(b->d_uexp.ptr, uexp.data(), uexp.size() * 4);
 }
 
 }  // namespace oj

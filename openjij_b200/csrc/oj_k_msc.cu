@@ -567,7 +567,7 @@ cudaError_t msc_prepare(oj_graph* g, int P, std::string* why) {
   auto put = [&](auto*& dst, const auto& vec, size_t bytes) -> cudaError_t {
     dst = reinterpret_cast<std::remove_reference_t<decltype(dst)>>(base + off);
     off += bytes;
-    return cudaMemcpy(dst, vec.data(), vec.size() * sizeof(vec[0]), cudaMemcpyHostToDevice);
+    return copy_tables(dst, vec.data(), vec.size() * sizeof(vec[0]));
   };
   if ((e = put(plan->gidx, gidx, b_gidx)) != cudaSuccess) return e;
   if ((e = put(plan->coff, coff, b_coff)) != cudaSuccess) return e;

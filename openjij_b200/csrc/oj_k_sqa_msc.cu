@@ -214,9 +214,9 @@ cudaError_t sqa_msc_prepare(oj_graph* g) {
   }
   cudaError_t e = g->sqa_nbr.ensure(std::max<size_t>(nbr.size() * 2, 16));
   if (e != cudaSuccess) return e;
-  if ((e = cudaMemcpy(g->sqa_nbr.ptr, nbr.data(), nbr.size() * 2, cudaMemcpyHostToDevice)) != cudaSuccess) return e;
+  if ((e = copy_tables(g->sqa_nbr.ptr, nbr.data(), nbr.size() * 2)) != cudaSuccess) return e;
   if ((e = g->sqa_jm.ensure(std::max<size_t>(jm.size() * 2, 16))) != cudaSuccess) return e;
-  return cudaMemcpy(g->sqa_jm.ptr, jm.data(), jm.size() * 2, cudaMemcpyHostToDevice);
+  return copy_tables(g->sqa_jm.ptr, jm.data(), jm.size() * 2);
 }
 
 cudaError_t launch_sqa_msc(const oj_graph* g, int R, int T, uint32_t* words, const uint32_t* thr,

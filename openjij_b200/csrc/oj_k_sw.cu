@@ -358,14 +358,14 @@ static cudaError_t sw_build(oj_graph* g) {
       quad[2 * b] = (uint32_t)ei[b] | ((uint32_t)ej[b] << 16);
       quad[2 * b + 1] = bits | (pos[b] ? 0u : 0x80000000u);
     }
-    e = cudaMemcpy(base + sw_array_bytes(ne), quad.data(), quad.size() * 4, cudaMemcpyHostToDevice);
+    e = copy_tables(base + sw_array_bytes(ne), quad.data(), quad.size() * 4);
     if (e != cudaSuccess) return e;
   }
   if (ne) {
-    if ((e = cudaMemcpy(base, ei.data(), ne * 4, cudaMemcpyHostToDevice)) != cudaSuccess) return e;
-    if ((e = cudaMemcpy(base + b_i, ej.data(), ne * 4, cudaMemcpyHostToDevice)) != cudaSuccess) return e;
-    if ((e = cudaMemcpy(base + 2 * b_i, w.data(), ne * 4, cudaMemcpyHostToDevice)) != cudaSuccess) return e;
-    if ((e = cudaMemcpy(base + 2 * b_i + b_w, pos.data(), ne, cudaMemcpyHostToDevice)) != cudaSuccess) return e;
+    if ((e = copy_tables(base, ei.data(), ne * 4)) != cudaSuccess) return e;
+    if ((e = copy_tables(base + b_i, ej.data(), ne * 4)) != cudaSuccess) return e;
+    if ((e = copy_tables(base + 2 * b_i, w.data(), ne * 4)) != cudaSuccess) return e;
+    if ((e = copy_tables(base + 2 * b_i + b_w, pos.data(), ne)) != cudaSuccess) return e;
   }
   g->sw_ne = (int64_t)ne;
   return cudaSuccess;

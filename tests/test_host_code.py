@@ -1,0 +1,105 @@
+"""The library's host code on the CPU, its objects linked against a stand-in
+for the CUDA runtime (fake/fake_cuda.cpp): the order of uploads and launches,
+what device memory a call takes and gives back, which kernel a call reaches.
+Kernels do not run, so spins stay as they are."""
+import ctypes as C
+import gc
+import glob
+import importlib.util
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from openjij_b200 import _native as N
+from openjij_b200 import instances as I
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="session")
+def fake_lib(tmp_path_factory):
+    spec = importlib.util.spec_from_file_location("_recipe", os.path.join(HERE, "..", "openjij_b200", "build.py"))
+    recipe = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(recipe)
+    recipe.build_cuda()
+    out = str(tmp_path_factory.mktemp("fake") / "libojb200_fake.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-Wl,-Bsymbolic",
+                    "-I" + os.path.join(os.path.dirname(recipe.NVCC), "..", "include"),
+                    os.path.join(HERE, "fake", "fake_cuda.cpp")] + sorted(glob.glob(recipe.BUILD + "/*.o")) +
+                   ["-o", out], check=True)
+    return out
+
+
+@pytest.fixture
+def fake(fake_lib):
+    """The library on the stand-in, in place of the real one; its context is fake.ctx."""
+    saved = N._lib, N.LIB_PATH
+    N._lib, N.LIB_PATH = None, fake_lib
+    lib = N.lib()
+    for name in ("fake_live_bytes", "fake_peak_bytes"):
+        getattr(lib, name).restype = C.c_size_t
+    lib.fake_launches.restype = C.c_char_p
+    lib.fake_fail_new.argtypes = [C.c_longlong, C.c_size_t]
+    lib.ctx = N.Context(0)
+    lib.fake_reset()
+    yield lib
+    lib.ctx.close()
+    gc.collect()
+    N._lib, N.LIB_PATH = saved
+
+
+def _chimera(ctx, cells, seed=1):
+    return N.Graph(ctx, *I.augmented_csr(I.chimera_pm_j(cells, seed=seed, field=0.5)[0]))
+
+
+def _lattice(ctx, side, seed=1):
+    return N.Graph(ctx, *I.augmented_csr(I.lattice_pm_j(side, seed=seed)[0]))
+
+
+def _first_sa(ctx, kernel, make):
+    g = make(ctx)
+    N.sa_run(g, np.ones((3, g.n), np.int8), [1.0], [2], seed=1, kernel=kernel, energies=np.zeros(3))
+
+
+def _first_sqa(ctx, kernel, make, T):
+    g = make(ctx)
+    N.sqa_run(g, np.ones((3, T, g.n), np.int8), 1.0, [1.0], [0.5], [2], seed=1, kernel=kernel)
+
+
+def _first_sw(ctx, make):
+    g = make(ctx)
+    N.sw_run(g, np.ones((3, g.n), np.int8), [1.0], [2], seed=1)
+
+
+def _first_batch(ctx):
+    mats = [I.dense_qubo_normal(n, seed=n)[0].toarray() for n in (40, 200)]
+    N.sa_run_batched(N.Batch(ctx, mats), [2, 3], np.ones(2 * 40 + 3 * 200, np.int8), [1.0], [2], seed=1)
+
+
+def _dense(ctx):
+    return N.Graph(ctx, *I.augmented_csr(I.dense_ising_uniform(90, seed=1)[0]))
+
+
+@pytest.mark.parametrize("call", [
+    lambda ctx: _first_sa(ctx, "colour", lambda c: _chimera(c, 6)),
+    lambda ctx: _first_sqa(ctx, "colour", lambda c: _chimera(c, 6), 5),
+    lambda ctx: _first_sa(ctx, "bitpacked", lambda c: _lattice(c, 16)),
+    lambda ctx: _first_sqa(ctx, "bitpacked", lambda c: _lattice(c, 16), 8),
+    lambda ctx: _first_sqa(ctx, "bitpacked", lambda c: _lattice(c, 16), 7),
+    lambda ctx: _first_sw(ctx, lambda c: _lattice(c, 40)),
+    lambda ctx: _first_sw(ctx, lambda c: _chimera(c, 4)),
+    lambda ctx: _first_sa(ctx, "dense_jump", _dense),
+    lambda ctx: _first_sa(ctx, "dense_plain", _dense),
+    lambda ctx: _first_sa(ctx, "dense_tc", _dense),
+    _first_batch,
+], ids=["sa colour", "sqa colour", "sa bit-packed", "sqa slice-split", "sqa bit-packed", "sw hooking", "sw",
+        "dense jump", "dense plain", "dense tc", "batch"])
+def test_tables_are_on_the_device_before_the_first_launch(fake, call):
+    """A graph's or batch's tables are uploaded by copies that may return
+    before the data is on the device; the context's stream does not wait for
+    them by itself."""
+    call(fake.ctx)
+    assert fake.fake_launches()
+    assert fake.fake_unordered() == 0
