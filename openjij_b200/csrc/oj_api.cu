@@ -529,6 +529,8 @@ oj_status oj_ctx_destroy(oj_ctx* ctx) {
     ctx->fields.release();
     ctx->eparts.release();
     ctx->counters.release();
+    ctx->fitems.release();
+    ctx->kstart.release();
     for (auto& e : ctx->ev)
       if (e) cudaEventDestroy(e);
     if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);

@@ -54,7 +54,8 @@ oj_graph::~oj_graph() {
   single_tab.release();
   sw_tables.release();
   if (cplan) cplan->tables.release();
-  if (msc) msc->tables.release();
+  msc.reset();
+  msc_other.clear();
   if (tc) {
     tc->bt_hi.release();
     tc->bt_lo.release();

@@ -24,10 +24,15 @@ inline std::atomic<long long>& alloc_fail_countdown() {
   return c;
 }
 
-// Grow-only device buffer owned by a context or graph.
+// Grow-only device buffer owned by a context or graph; freed with its owner,
+// so that tables whose build fails half way are given back.
 struct DevBuf {
   void* ptr = nullptr;
   size_t bytes = 0;
+  DevBuf() = default;
+  DevBuf(const DevBuf&) = delete;
+  DevBuf& operator=(const DevBuf&) = delete;
+  ~DevBuf() { release(); }
   cudaError_t ensure(size_t want) {
     if (want <= bytes) return cudaSuccess;
     if (alloc_fail_countdown().load() >= 0 && alloc_fail_countdown().fetch_sub(1) == 0)
@@ -144,6 +149,9 @@ struct oj_graph {
   oj::DevBuf d_rp, d_ci, d_val, d_h, d_val64, d_h64, d_order, d_coff;
   oj::DevBuf d_dense;  // FP32 dense J (n x n), created on first use
   std::unique_ptr<oj::MscPlan> msc;
+  // the plans of other cluster sizes that earlier calls took: kept, since a run of
+  // another context may still read one (at most one for each size)
+  std::vector<std::unique_ptr<oj::MscPlan>> msc_other;
   std::unique_ptr<oj::TcPlan> tc;
   oj::DevBuf sqa_nbr, sqa_jm;  // bit-packed SQA tables: [n][D] neighbours (u16), [n] J>0 masks
   std::map<uint64_t, oj::Shape> tuned;  // autotuned launch shapes by (kernel, replicas, slices)

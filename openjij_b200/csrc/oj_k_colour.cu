@@ -567,10 +567,7 @@ static cudaError_t colour_build(oj_graph* g) {
   std::memcpy(host.data() + b_site, cls.data(), cls.size() * 16);
   std::memcpy(host.data() + b_site + b_cls, slice.data(), slice.size() * 8);
   std::memcpy(host.data() + b_site + b_cls + b_slice, ent.data(), ent.size() * 8);
-  if ((e = copy_tables(base, host.data(), host.size())) != cudaSuccess) {
-    plan->tables.release();
-    return e;
-  }
+  if ((e = copy_tables(base, host.data(), host.size())) != cudaSuccess) return e;
   g->cplan = std::move(plan);
   return cudaSuccess;
 }

@@ -424,6 +424,11 @@ int msc_choose_cluster(const oj_graph* g, int G, int sm_count) {
 // Host-side partition of the sites over the P CTAs of a cluster.
 cudaError_t msc_prepare(oj_graph* g, int P, std::string* why) {
   if (g->msc && g->msc->P == P) return cudaSuccess;
+  for (auto& other : g->msc_other)
+    if (other->P == P) {
+      std::swap(g->msc, other);
+      return cudaSuccess;
+    }
   const int n = g->n;
   const int D = g->info.max_degree;
   const int ncol = g->info.num_colours;
@@ -579,6 +584,7 @@ cudaError_t msc_prepare(oj_graph* g, int P, std::string* why) {
   if ((e = put(plan->jm, jm, b_jm)) != cudaSuccess) return e;
   if ((e = put(plan->poff, poff, b_poff)) != cudaSuccess) return e;
   if ((e = put(plan->pent, pent, b_pent)) != cudaSuccess) return e;
+  if (g->msc) g->msc_other.push_back(std::move(g->msc));
   g->msc = std::move(plan);
   return cudaSuccess;
 }

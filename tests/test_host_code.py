@@ -103,3 +103,69 @@ def test_tables_are_on_the_device_before_the_first_launch(fake, call):
     call(fake.ctx)
     assert fake.fake_launches()
     assert fake.fake_unordered() == 0
+
+
+def test_a_failing_host_allocation_of_the_colour_tables_leaks_no_device_memory(fake):
+    """Every host allocation of the first run's table build fails in turn: the
+    run is out of memory, the graph is usable, and destroying both gives all
+    device memory back."""
+    n = 40000
+    i = np.arange(n)
+    m = I.augmented_from_ising(np.full(n, 0.25), (np.minimum(i, (i + 1) % n), np.maximum(i, (i + 1) % n), i % 7 + 1.0), n)
+    aug = I.augmented_csr(m)
+    fake.ctx.close()
+    for k in range(100):
+        before = fake.fake_live_bytes()
+        ctx = N.Context(0)
+        g = N.Graph(ctx, *aug)
+        s = np.ones((1, n), np.int8)
+        fake.fake_fail_new(k, 64 * 1024)
+        try:
+            N.sa_run(g, s, [1.0], [1], seed=1, kernel="colour")
+        except N.OJError as err:
+            assert err.status == N.OJ_ERR_OOM
+        done = fake.fake_new_pending()
+        fake.fake_fail_new(-1, 0)
+        N.sa_run(g, s, [1.0], [1], seed=1, kernel="colour")
+        g.close()
+        ctx.close()
+        if k > 0:  # the first context sets up what the process keeps
+            assert fake.fake_live_bytes() == before, k
+        if done:
+            break
+    assert 0 < k < 99
+
+
+def test_plans_of_several_cluster_sizes_are_bounded_and_given_back(fake):
+    """The number of replicas sets the cluster size of the bit-packed kernel;
+    calls that alternate it build each size's plan once."""
+    fake.ctx.close()
+    ctx = N.Context(0)
+    before = fake.fake_live_bytes()
+    g = _lattice(ctx, 72)
+    sizes = set()
+    for turn in range(3):
+        for R in (32, 640, 1600):
+            sizes.add(N.sa_run(g, np.ones((R, g.n), np.int8), [1.0], [1], seed=1, kernel="bitpacked")["cluster"])
+        live = fake.fake_live_bytes()
+        assert turn == 0 or live == first
+        first = live
+    assert len(sizes) > 1
+    g.close()
+    ctx.close()
+    assert fake.fake_live_bytes() <= before
+
+
+def test_a_context_gives_back_its_buffers(fake):
+    fake.ctx.close()
+    before = fake.fake_live_bytes()
+    ctx = N.Context(0)
+    g = _dense(ctx)
+    b = N.Batch(ctx, [I.dense_qubo_int(200, seed=1)[0].toarray()])
+    N.sa_run(g, np.ones((3, g.n), np.int8), [1.0], [2], seed=1, energies=np.zeros(3))
+    N.sa_run_batched(b, [40], np.ones(40 * 200, np.int8), [1.0], [2], seed=1, energies=np.zeros(40))
+    N.sqa_run(g, np.ones((3, 4, g.n), np.int8), 1.0, [1.0], [0.5], [2], seed=1, energies=np.zeros((3, 4)))
+    b.close()
+    g.close()
+    ctx.close()
+    assert fake.fake_live_bytes() <= before
