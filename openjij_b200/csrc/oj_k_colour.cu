@@ -282,8 +282,9 @@ __global__ void __launch_bounds__(kColourThreads) sqa_colour_kernel(ColourArgs a
   ojd::add_flips(a.flips, nflip);
 }
 
-// SA on graphs whose spins do not fit shared memory (updated in place in global
-// memory).  One CTA per replica quad q (replicas 4q..4q+3); one thread per
+// SA on graphs whose spins do not fit shared memory, or whose tables
+// (ColourPlan) there is no room for; the spins are updated in place in global
+// memory.  One CTA per replica quad q (replicas 4q..4q+3); one thread per
 // (site, quad): the four replicas share the neighbour loads and one Philox call.
 __global__ void __launch_bounds__(kColourGlobalThreads)
     sa_colour_global_kernel(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
@@ -573,8 +574,9 @@ static cudaError_t colour_build(oj_graph* g) {
 }
 
 // Builds the graph's ColourPlan (once).  No exception leaves it: its callers
-// are reached through the C interface, and a host allocation that fails is
-// reported as out of memory.
+// are reached through the C interface.  A host or device allocation that fails
+// is reported as out of memory, and so are lists that pad to more entries than
+// an int counts; the run then takes the kernels that read the graph's own lists.
 cudaError_t colour_prepare(oj_graph* g) {
   const std::lock_guard<std::mutex> lock(g->cplan_lock);
   if (g->cplan) return cudaSuccess;
@@ -635,16 +637,19 @@ cudaError_t launch_sa_colour(const oj_graph* g, int R, int8_t* spins, const floa
                              int64_t nsweeps, RngBase rb, cudaStream_t st, int* launches) {
   if (seq_applies(g, 1)) return launch_sa_seq(g, R, spins, betas, nsweeps, rb, st, launches);
   if (launches) ++*launches;
-  if (g->n > kSmemBudget) {
+  const bool fits = g->n <= kSmemBudget;
+  const cudaError_t pe = fits ? colour_prepare(const_cast<oj_graph*>(g)) : cudaSuccess;
+  if (!fits || pe == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
     sa_colour_global_kernel<<<(R + 3) / 4, kColourGlobalThreads, 0, st>>>(
         g->d_rp.as<int32_t>(), g->d_ci.as<int32_t>(), g->d_val.as<float>(), g->d_h.as<float>(),
         g->d_order.as<int32_t>(), g->d_coff.as<int32_t>(), g->info.num_colours, g->n, R, spins, betas, nsweeps, rb);
     return cudaGetLastError();
   }
+  if (pe != cudaSuccess) return pe;
   int sms = 0;
-  cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device);
+  const cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device);
   if (e != cudaSuccess) return e;
-  if ((e = colour_prepare(const_cast<oj_graph*>(g))) != cudaSuccess) return e;
   ColourArgs a = colour_args(g, R, 1, spins, nsweeps, rb);
   a.betas = betas;
   // eight replicas a CTA share the neighbour entries; four where that leaves
@@ -666,16 +671,19 @@ cudaError_t launch_sqa_colour(const oj_graph* g, int R, int T, int8_t* spins, co
   if (launches) ++*launches;
   const int octets = (T + 7) / 8;
   const size_t smem = (size_t)octets * g->n;
-  if (smem > (size_t)kSmemBudget) {
+  const bool fits = smem <= (size_t)kSmemBudget;
+  const cudaError_t pe = fits ? colour_prepare(const_cast<oj_graph*>(g)) : cudaSuccess;
+  if (!fits || pe == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
     sqa_colour_global_kernel<<<R, kSqaGlobalThreads, 0, st>>>(
         g->d_rp.as<int32_t>(), g->d_ci.as<int32_t>(), g->d_val.as<float>(), g->d_h.as<float>(),
         g->d_order.as<int32_t>(), g->d_coff.as<int32_t>(), g->info.num_colours, g->n, T, spins, coef, nsweeps, rb);
     return cudaGetLastError();
   }
+  if (pe != cudaSuccess) return pe;
   int sms = 0;
-  cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device);
+  const cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device);
   if (e != cudaSuccess) return e;
-  if ((e = colour_prepare(const_cast<oj_graph*>(g))) != cudaSuccess) return e;
   ColourArgs a = colour_args(g, R, T, spins, nsweeps, rb);
   a.coef = coef;
   const int threads = colour_threads((int64_t)octets * ((g->cplan->max_class + 31) / 32 * 32), R, sms);

@@ -169,3 +169,45 @@ def test_a_context_gives_back_its_buffers(fake):
     g.close()
     ctx.close()
     assert fake.fake_live_bytes() <= before
+
+
+@pytest.mark.parametrize("failing", ["device", "host"])
+def test_a_colour_run_without_room_for_its_tables_reads_the_neighbour_lists(fake, failing):
+    """The tables of the shared-memory colour kernels are only there for speed:
+    where they cannot be allocated, the run takes the kernels that read the
+    graph's own lists, as one too large for shared memory does."""
+    n = 40000
+    i = np.arange(n)
+    m = I.augmented_from_ising(np.full(n, 0.25), (np.minimum(i, (i + 1) % n), np.maximum(i, (i + 1) % n), i % 7 + 1.0), n)
+    g = N.Graph(fake.ctx, *I.augmented_csr(m))
+    s = np.ones((1, 3, n), np.int8)
+
+    def sa():
+        N.sa_run(g, s[:, 0], [1.0], [1], seed=1, kernel="colour")
+
+    def sqa():
+        N.sqa_run(g, s, 1.0, [1.0], [0.5], [1], seed=1, kernel="colour")
+
+    N.sw_run(g, s[:, 0], [1.0], [1], seed=1, energies=np.zeros(1))  # sizes the context's buffers
+    fake.ctx.inject_alloc_failure(10**6)
+    for run, kernel in ((sa, b"sa_colour_global_kernel"), (sqa, b"sqa_colour_global_kernel")):
+        for k in range(20):
+            fake.fake_reset()
+            if failing == "host":
+                fake.fake_fail_new(k, 64 * 1024)
+            else:
+                fake.ctx.inject_alloc_failure(k)
+            try:
+                run()
+            except N.OJError as err:  # a buffer of the call itself
+                assert err.status == N.OJ_ERR_OOM
+            else:
+                if fake.fake_launches().count(kernel):
+                    break
+        else:
+            raise AssertionError("no failing allocation reached " + kernel.decode())
+        fake.fake_fail_new(-1, 0)
+        fake.ctx.inject_alloc_failure(None)
+    fake.fake_reset()
+    sa()  # with room again the tables are built
+    assert b"global" not in fake.fake_launches()
