@@ -384,7 +384,6 @@ cudaError_t launch_energy(const oj_graph* g, int count, const int8_t* spins, dou
 cudaError_t launch_best_slice(const double* energies, int R, int T, int32_t* best, cudaStream_t st);
 
 // Kernel limits used by the planner.
-int sa_colour_max_smem_sites();
 int msc_max_degree();
 int msc_default_threads(const oj_graph* g, int P);
 int cluster_most(int G);

@@ -508,8 +508,6 @@ __global__ void unpack_kernel(const uint32_t* __restrict__ words, int R, int n, 
 
 }  // namespace
 
-int sa_colour_max_smem_sites() { return kSmemBudget; }
-
 static cudaError_t colour_build(oj_graph* g) {
   const int n = g->n, ncol = g->info.num_colours;
   std::vector<int32_t> order(g->order), slot(n);
