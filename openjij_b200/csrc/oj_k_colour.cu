@@ -30,7 +30,13 @@
 namespace oj {
 namespace {
 
-constexpr int kColourThreads = 1024;       // most threads of a CTA with the spins in shared memory
+// Most threads of a CTA with the spins in shared memory.  An SM has 1024 at work
+// (colour_threads), so the kernels ask for one CTA an SM of this size, 64 registers a
+// thread; with the bound of threads alone the compiler took 32, which put the loads
+// of a neighbour list one after another (300 sites of mean degree 90, 31 classes, us a
+// sweep: SA with 8 replicas 577, now 114; SQA with 2 slices 692, now 195; 300 sites of
+// degree 4, SA with 8 replicas 9.5, now 6.5).
+constexpr int kColourThreads = 1024;
 constexpr int kColourGlobalThreads = 256;  // SA with the spins in global memory
 constexpr int kSqaGlobalThreads = 512;     // SQA with the spins in global memory
 constexpr int kSmemBudget = 200 * 1024;
@@ -96,7 +102,7 @@ __device__ __forceinline__ void colour_fields(const int2* __restrict__ ent, int 
 // to tell (neglog_gap).  Chimera lattice of 2048
 // sites with fields, 1024 replicas, 1000 sweeps: 11.97 -> 5.02 ms (56 instructions an attempt, ALU pipe 63 %).
 template <int NQ, bool LONG>
-__global__ void __launch_bounds__(kColourThreads) sa_colour_kernel(ColourArgs a) {
+__global__ void __launch_bounds__(kColourThreads, 1) sa_colour_kernel(ColourArgs a) {
   extern __shared__ uint8_t S[];  // [n] by slot
   constexpr int NF = 4 * NQ;
   const int r0 = NF * blockIdx.x, nr = min(NF, a.R - r0);
@@ -181,7 +187,7 @@ __global__ void __launch_bounds__(kColourThreads) sa_colour_kernel(ColourArgs a)
 // steps as the SA kernel above.  Chimera lattice of 512 sites,
 // 8 slices, 128 replicas, 500 sweeps: 5.11 -> 1.94 ms.
 template <int NJ, bool LONG>
-__global__ void __launch_bounds__(kColourThreads) sqa_colour_kernel(ColourArgs a) {
+__global__ void __launch_bounds__(kColourThreads, 1) sqa_colour_kernel(ColourArgs a) {
   extern __shared__ uint8_t S[];  // [octets][n] by slot
   const int r = blockIdx.x;
   const int n = a.n, T = a.T, no = (T + 7) >> 3;
