@@ -753,12 +753,15 @@ oj_status oj_sa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int8_t* spins, c
     // the cached shape's cluster when there is one, so the plan is built once
     const uint64_t key = ((uint64_t)OJ_KERNEL_BITPACKED << 40) | (uint64_t)R;
     const auto cached = g->tuned.find(key);
-    const int P = (cached != g->tuned.end() && cached->second.cluster) ? cached->second.cluster
-                                                                       : msc_choose_cluster(g, G, ctx->sm_count);
-    cudaError_t pe = msc_prepare(g, P, &why);
+    cudaError_t pe = msc_prepare_from(g,
+                                      cached != g->tuned.end() && cached->second.cluster
+                                          ? cached->second.cluster
+                                          : msc_choose_cluster(g, G, ctx->sm_count),
+                                      &why);
     if (pe != cudaSuccess) {
       return prep_fail(ctx, pe, why);
     }
+    const int P = g->msc->P;
     std::vector<uint32_t> thr, alw;
     msc_thresholds(bf, inf.coupling_abs, D, thr, alw);
     const size_t pbytes = (thr.size() + alw.size()) * 4;
@@ -785,9 +788,7 @@ oj_status oj_sa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int8_t* spins, c
           for (int th : {256, 512, 1024}) cand.push_back(Shape{Pc, th, 0});
       int def_msc = -1;  // the heuristic shape
       for (size_t q = 0; q < cand.size(); ++q)
-        if (cand[q].cluster == msc_choose_cluster(g, G, ctx->sm_count) &&
-            cand[q].threads == msc_default_threads(g, cand[q].cluster))
-          def_msc = (int)q;
+        if (cand[q].cluster == P && cand[q].threads == msc_default_threads(g, cand[q].cluster)) def_msc = (int)q;
       OJ_CK(ctx->aux.ensure((size_t)G * n * 4), "alloc tuning scratch");
       uint32_t* scratch = ctx->aux.as<uint32_t>();
       const int64_t Ssub = std::min<int64_t>(S, 16);
@@ -807,7 +808,7 @@ oj_status oj_sa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int8_t* spins, c
       g->tuned[key] = shp;
       tuned_now = true;
     }
-    P_used = shp.cluster ? shp.cluster : msc_choose_cluster(g, G, ctx->sm_count);
+    P_used = shp.cluster ? shp.cluster : P;
     threads_used = shp.threads ? shp.threads : msc_default_threads(g, P_used);
     pe = msc_prepare(g, P_used, &why);
     if (pe != cudaSuccess) {

@@ -390,6 +390,7 @@ int cluster_most(int G);
 int split_default_threads(const oj_graph* g, int P);
 int largest_class(const oj_graph* g);
 cudaError_t msc_prepare(oj_graph* g, int P, std::string* why);
+cudaError_t msc_prepare_from(oj_graph* g, int P, std::string* why);
 int msc_choose_cluster(const oj_graph* g, int G, int sm_count);
 
 }  // namespace oj

@@ -589,6 +589,17 @@ cudaError_t msc_prepare(oj_graph* g, int P, std::string* why) {
   return cudaSuccess;
 }
 
+// The plan of cluster size P, or of the next larger one whose parts with their
+// halos fit shared memory (msc_choose_cluster only estimates the halos).
+cudaError_t msc_prepare_from(oj_graph* g, int P, std::string* why) {
+  cudaError_t e = msc_prepare(g, P, why);
+  while (e == cudaErrorInvalidValue && P < kMscMaxCluster) {
+    if (why) why->clear();
+    e = msc_prepare(g, ++P, why);
+  }
+  return e;
+}
+
 cudaError_t launch_sa_msc(const oj_graph* g, int G, uint32_t* words, const uint32_t* thr,
                           const uint32_t* always, int64_t nsweeps, RngBase rb, cudaStream_t st,
                           int* launches, int threads) {

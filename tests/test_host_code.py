@@ -211,3 +211,23 @@ def test_a_colour_run_without_room_for_its_tables_reads_the_neighbour_lists(fake
     fake.fake_reset()
     sa()  # with room again the tables are built
     assert b"global" not in fake.fake_launches()
+
+
+def _circulant(ctx, n, degree, seed=1):
+    """+-J couplings to the sites at degree / 2 random offsets on either side: a
+    regular graph on which every part of a partition borders most others."""
+    rng = np.random.default_rng(seed)
+    i = np.arange(n)
+    a = np.tile(i, degree // 2)
+    b = np.concatenate([(i + k) % n for k in rng.choice(np.arange(1, n // 2), degree // 2, replace=False)])
+    m = I.augmented_from_ising(np.zeros(n), (np.minimum(a, b), np.maximum(a, b), rng.choice([-1.0, 1.0], a.size)), n)
+    return N.Graph(ctx, *I.augmented_csr(m))
+
+
+@pytest.mark.parametrize("n,degree,R", [(40000, 8, 400), (60000, 6, 32), (30000, 8, 400)])
+def test_bitpacked_runs_take_a_cluster_that_their_partition_fits(fake, n, degree, R):
+    """The number of CTAs a group gets follows the number of groups; the halos of
+    a graph without locality may need more of them."""
+    g = _circulant(fake.ctx, n, degree)
+    st = N.sa_run(g, np.ones((R, n), np.int8), [1.0], [1], seed=1, kernel="bitpacked")
+    assert st["cluster"] <= 16
