@@ -1811,11 +1811,11 @@ oj_status oj_sw_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int8_t* spins, c
   float* d_beta = ctx->params.as<float>();
   if (S > 0) OJ_CK(cudaMemcpyAsync(d_beta, bf.data(), bf.size() * 4, cudaMemcpyHostToDevice, st), "H2D betas");
   OJ_CK(cudaEventRecord(ctx->ev[1], st), "event");
-  // graphs above the shared-memory size keep the parent links of a chunk of
+  // graphs whose parent links do not fit shared memory keep those of a chunk of
   // replicas in global scratch (at most 1 GiB)
   uint32_t* scratch = nullptr;
   int chunk = 0;
-  if (n > sw_max_sites()) {
+  if (sw_needs_scratch(g, R, ctx->sm_count)) {
     const size_t per = ((size_t)n + 1) * 4;
     chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)R, ((size_t)1 << 30) / per));
     OJ_CK(ctx->aux.ensure(per * (size_t)chunk), "alloc union-find scratch");

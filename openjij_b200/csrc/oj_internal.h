@@ -277,6 +277,8 @@ cudaError_t launch_sqa_split_unpack(const uint32_t* words, int R, int T, int n, 
 size_t sw_smem_bytes(int n);
 int sw_max_sites();
 int sw_threads(const oj_graph* g, int R, int sm_count);  // after sw_prepare
+// The run keeps its parent links in global scratch (after sw_prepare).
+bool sw_needs_scratch(const oj_graph* g, int R, int sm_count);
 cudaError_t sw_prepare(oj_graph* g);
 cudaError_t launch_sw(const oj_graph* g, int R, int8_t* spins, const float* betas, int64_t nsweeps, RngBase rb,
                       uint32_t* scratch, int chunk, int sm_count, cudaStream_t st, int* launches);

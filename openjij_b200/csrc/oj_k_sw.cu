@@ -322,6 +322,10 @@ int sw_threads(const oj_graph* g, int R, int sm_count) {
   return sw_hooks(g, R, sm_count) && R <= sm_count ? kSwHookThreads : kSwThreads;
 }
 
+bool sw_needs_scratch(const oj_graph* g, int R, int sm_count) {
+  return g->n > sw_max_sites() && !sw_hooks(g, R, sm_count);
+}
+
 // Bond list of the graph: (i, j) with i < j from the neighbour lists, then
 // (i, n) for every non-zero h_i.
 static cudaError_t sw_build(oj_graph* g) {
@@ -387,7 +391,8 @@ cudaError_t launch_sw(const oj_graph* g, int R, int8_t* spins, const float* beta
   const int n = g->n;
   const bool in_smem = n <= sw_max_sites();
   const size_t smem = in_smem ? sw_smem_bytes(n) : 0;
-  if (g->sw_ne > (int64_t)0x7FFFFFFF || (!in_smem && (!scratch || chunk < 1))) return cudaErrorInvalidValue;
+  if (g->sw_ne > (int64_t)0x7FFFFFFF || (sw_needs_scratch(g, R, sm_count) && (!scratch || chunk < 1)))
+    return cudaErrorInvalidValue;
   const int64_t ne = g->sw_ne;
   const size_t b_i = sw_align((size_t)ne * 4 + 4), b_w = sw_align((size_t)ne * 4 + 4);
   const char* base = g->sw_tables.as<char>();

@@ -44,3 +44,16 @@ def test_swendsen_wang_hooking_lattice_bit_exact(ctx):
     st = N.sw_run(dg, s, betas, mcs, seed=62)
     np.testing.assert_array_equal(s, O.replay_sw(g, s0, np.repeat(betas, mcs).astype(np.float32), 62))
     assert st["threads"] == 1024
+
+
+@pytest.mark.parametrize("side", [212, 214, 216, 218])
+def test_swendsen_wang_around_the_shared_memory_limits_bit_exact(ctx, side):
+    """Sides on either side of both kernels' shared-memory limits; only the last
+    keeps its links in global scratch."""
+    g = O.AugCSR(I.lattice_pm_j(side, seed=4)[0])
+    dg = N.Graph(ctx, g.n, g.indptr, g.indices, g.data)
+    betas = np.array([0.3, 2.0])
+    s0 = np.random.default_rng(side).choice(np.array([-1, 1], np.int8), size=(2, g.n))
+    s = s0.copy()
+    N.sw_run(dg, s, betas, np.ones(2, np.int32), seed=63)
+    np.testing.assert_array_equal(s, O.replay_sw(g, s0, betas.astype(np.float32), 63))

@@ -231,3 +231,18 @@ def test_bitpacked_runs_take_a_cluster_that_their_partition_fits(fake, n, degree
     g = _circulant(fake.ctx, n, degree)
     st = N.sa_run(g, np.ones((R, n), np.int8), [1.0], [1], seed=1, kernel="bitpacked")
     assert st["cluster"] <= 16
+
+
+def test_swendsen_wang_takes_union_find_scratch_only_for_the_kernel_that_uses_it(fake):
+    """A lattice of side 214 has more sites than the walking kernel holds in
+    shared memory, but the hooking kernel takes it; side 230 fits neither."""
+    for side, kernel, needs in ((214, b"sw_hook_kernel", False), (230, b"sw_kernel", True)):
+        g = _lattice(fake.ctx, side)
+        R = 100
+        fake.fake_reset()
+        before = fake.fake_live_bytes()
+        N.sw_run(g, np.ones((R, g.n), np.int8), [1.0], [1], seed=1)
+        assert kernel in fake.fake_launches()
+        forest = 4 * R * (g.n + 1)
+        assert (fake.fake_live_bytes() - before >= forest) == needs
+        g.close()
