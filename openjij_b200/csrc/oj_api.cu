@@ -832,7 +832,7 @@ oj_status oj_sa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int8_t* spins, c
     };
     const uint64_t key = ((uint64_t)OJ_KERNEL_DENSE_JUMP << 40) | (uint64_t)R;
     auto tit = g->tuned.find(key);
-    int variant = tit != g->tuned.end() ? tit->second.variant : batch_default_variant(n, R, ctx->sm_count);
+    int variant = tit != g->tuned.end() ? tit->second.variant : batch_default_variant(1, &n, &R, ctx->sm_count);
     if (n > batch_variant_max_n(variant)) variant = 83;
     std::vector<int32_t> items = make_items(batch_variant_warps(variant));
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
@@ -1618,7 +1618,7 @@ oj_status oj_sa_run_batched(oj_ctx* ctx, const oj_batch* b, const int32_t* reads
     return it;
   };
   oj_batch* bm = const_cast<oj_batch*>(b);
-  int variant0 = bm->tuned_variant ? bm->tuned_variant : batch_default_variant(b->max_n, nrep, ctx->sm_count);
+  int variant0 = bm->tuned_variant ? bm->tuned_variant : batch_default_variant(count, b->n.data(), reads, ctx->sm_count);
   if (b->max_n > batch_variant_max_n(variant0)) variant0 = 83;
   std::vector<int32_t> items = make_items(batch_variant_warps(variant0));
   const size_t items_cap = make_items(batch_min_warps()).size();  // the most items of any variant

@@ -286,7 +286,7 @@ int batch_max_sites();
 int batch_warps();
 int batch_variant_warps(int variant);
 int batch_min_warps();  // fewest warps per CTA of any variant (most work items)
-int batch_default_variant(int max_n, int64_t replicas, int sm_count);
+int batch_default_variant(int count, const int32_t* n, const int32_t* reads, int sm_count);
 int batch_variant_max_n(int variant);  // largest instance a launch variant takes
 // Tensor-core local fields of a batch (oj_k_field_tc.cu).
 struct FieldCall {

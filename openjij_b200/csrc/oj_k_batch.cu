@@ -41,6 +41,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
 
 #include "oj_device.cuh"
@@ -670,17 +671,40 @@ int batch_variant_max_n(int variant) {
 // Batches of up to 512 sites (four chunks) take variant 83: a flip row is one
 // group of loads, and more warps hide it.  Larger instances take 45, which has
 // eight chunks' loads in flight: 2048 sites, 4096 replicas, 1000 sweeps 21.9
-// (83), 22.3 (82), 20.0 ms (45); 520 to 2048 sites with 8 to 4096 replicas 2 to 24 %
-// less; 64 instances of 64 to 512 sites with 32 reads 6.4 (83), 7.1 ms (45).  One-chunk
-// batches with at most eight replicas an SM spread them over more CTAs of four warps
-// (100 sites, 100 reads, 1000 sweeps 2.17 (83), 1.94 ms (45)).
-int batch_default_variant(int max_n, int64_t replicas, int sm_count) {
+// (83), 22.3 (82), 20.7 ms (45); 520 to 2048 sites with 1024 or 4096 replicas 3 to
+// 16 % less; 64 instances of 64 to 1024 sites with 1 to 64 reads 4 to 30 % less; 64 instances
+// of 64 to 512 sites with 32 reads 6.4 (83), 7.1 ms (45).  But 83 holds 24 replicas an SM
+// and 45 only 20, so 83 is faster again
+//   * for equal replicas, all of which run at once only there (3000 replicas, 200
+//     sweeps, 45 / 83: 520 sites 5.08 / 4.59 ms, 1500 sites 13.97 / 13.00), and, where
+//     45's second group of loads is half empty (9 to 12 chunks), from 12 an SM on (2048
+//     replicas: 1300 sites 8.46 / 8.13, 1500 sites 9.43 / 9.13);
+//   * where the SMs are full (40 replicas an SM) and enough of the replicas are of
+//     the small instances (22 an SM) to fill them at the end: 200 sweeps, 200 instances of
+//     100 to 700 sites with 24 reads 5.97 / 6.15, 32 reads 7.30 / 6.76, 64 reads 13.25 /
+//     12.06; 512 of 64 to 1024 sites with 12 reads 11.20 / 11.84, 16 reads 13.42 / 13.09, 64
+//     reads 42.99 / 41.14.
+// One-chunk batches with at most eight replicas an SM spread them over more CTAs of
+// four warps (100 sites, 100 reads, 1000 sweeps 2.17 (83), 1.94 ms (45)).
+int batch_default_variant(int count, const int32_t* n, const int32_t* reads, int sm_count) {
   if (const char* env = std::getenv("OJ_BATCH_VARIANT")) {
     const int v = std::atoi(env);
     if (batch_variant_valid(v)) return v;
   }
-  if (max_n <= 128) return replicas <= 8 * (int64_t)sm_count ? 45 : 83;
-  return max_n > 512 ? 45 : 83;
+  int64_t replicas = 0, small = 0, sms = sm_count;
+  int lo = INT_MAX, hi = 0;  // sites of the instances with reads
+  for (int k = 0; k < count; ++k) {
+    hi = std::max(hi, n[k]);
+    if (reads[k] == 0) continue;
+    lo = std::min(lo, n[k]);
+    replicas += reads[k];
+    if (n[k] <= 512) small += reads[k];
+  }
+  if (hi <= 128) return replicas <= 8 * sms ? 45 : 83;
+  if (hi <= 512) return 83;
+  const int chunks = (hi + 127) / 128;
+  if (lo == hi && replicas <= 24 * sms && replicas > (chunks >= 9 && chunks <= 12 ? 12 : 20) * sms) return 83;
+  return replicas >= 40 * sms && small >= 22 * sms ? 83 : 45;
 }
 
 template <int W, int MINB, int GROUP>

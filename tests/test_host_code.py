@@ -246,3 +246,22 @@ def test_swendsen_wang_takes_union_find_scratch_only_for_the_kernel_that_uses_it
         forest = 4 * R * (g.n + 1)
         assert (fake.fake_live_bytes() - before >= forest) == needs
         g.close()
+
+
+@pytest.mark.parametrize("sizes,reads,variant", [
+    (np.linspace(100, 700, 200), 24, 45), (np.linspace(100, 700, 200), 32, 83),
+    (np.linspace(64, 1024, 512), 12, 45), (np.linspace(64, 1024, 512), 16, 83),
+    ([777], 2960, 45), ([777], 2961, 83), ([777], 3553, 45), ([1300], 2048, 83), ([1300], 1776, 45),
+    ([2048], 4096, 45), ([512], 4096, 83)])
+def test_default_variant_of_large_instances(fake, sizes, reads, variant):
+    """More than 512 sites: the variant with more loads in flight, except where
+    the one with more replicas an SM runs them in fewer turns."""
+    sizes = np.asarray(sizes, int)
+    b = N.Batch(fake.ctx, [np.pad([[1.0]], ((n, 0), (n, 0))) for n in sizes])
+    st = N.sa_run_batched(b, np.full(len(sizes), reads, np.int32), np.ones(int(sizes.sum()) * reads, np.int8), [1.0],
+                          [1], seed=1)
+    assert st["variant"] == variant
+    if len(sizes) == 1:
+        g = N.Graph(fake.ctx, *I.augmented_csr(I.dense_qubo_int(int(sizes[0]), seed=1)[0]))
+        st = N.sa_run(g, np.ones((reads, g.n), np.int8), [1.0], [1], seed=1, kernel="dense_jump")
+        assert st["variant"] == variant
