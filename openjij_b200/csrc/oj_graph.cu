@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <string>
 #include <vector>
 
@@ -278,6 +279,15 @@ oj_status finish_graph(oj_ctx* ctx, oj_graph* g) {
   {
     std::vector<int32_t> fill(g->coff.begin(), g->coff.end() - 1);
     for (int i = 0; i < n; ++i) g->order[fill[g->colour[i]]++] = i;
+  }
+  {
+    double span = 0.0;
+    for (int i = 0; i < n; ++i)
+      for (int q = g->rp[i]; q < g->rp[i + 1]; ++q) {
+        const int d = std::abs(g->ci[q] - i);
+        span += std::min(d, n - d);
+      }
+    g->local = 16.0 * span <= (double)n * (double)g->ci.size();
   }
   // device copies
   cudaError_t e;

@@ -145,6 +145,7 @@ struct oj_graph {
   std::vector<int32_t> colour, order, coff;  // greedy colouring; sites sorted by colour
   oj_graph_info info{};
   bool regular = false;
+  bool local = false;  // neighbours' indices differ, on average, by at most n / 16 (counted round the end)
   // device copies
   oj::DevBuf d_rp, d_ci, d_val, d_h, d_val64, d_h64, d_order, d_coff;
   oj::DevBuf d_dense;  // FP32 dense J (n x n), created on first use

@@ -309,11 +309,23 @@ size_t sw_array_bytes(size_t ne) { return 2 * sw_align(ne * 4 + 4) + sw_align(ne
 // The graph has quads: its sites are 16-bit indices and its state fits.
 bool sw_has_quads(int n, size_t ne) { return n < 65535 && sw_hook_smem(n, (ne + 3) / 4) <= kSwHookSmemBytes; }
 
-// The hooking kernel (figures there) from 8192 sites on, from 2048 on with at most two
-// replicas an SM, and from 1024 on where every replica has an SM to itself (1024
-// threads each).
+// Where the hooking kernel is the faster one (us a sweep of a 30-sweep call, energies
+// included, sw_kernel / it).  A replica that has an SM to itself (1024 threads): from
+// 1024 sites and 2100 bonds on (148 replicas: lattices of 32 x 32, 2048 bonds 5.8 / 6.5, and
+// 33 x 33, 2178 bonds 7.8 / 7.0; 3-regular 1300 sites, 1950 bonds 6.6 / 7.2, 1400 sites
+// 7.9 / 7.3).  With several replicas an SM sw_kernel's walks overlap, and they are
+// short unless neighbours are near in index order, which makes long chains of sites:
+// from 8192 such sites on, and with two replicas an SM from 2048 sites and 6500 bonds on
+// (lattices with 256 replicas: 46 x 46 13.6 / 15.7, 56 x 56 20.2 / 20.7, 64 x 64 26.2 /
+// 25.0; 1024 replicas: 64 x 64 69 / 71, 91 x 91 152 / 140); without that order only from
+// 40000 sites on (3-regular, 1024 replicas: 8200 sites 104 / 122, 20000 sites 311 / 332,
+// 40000 sites 941 / 911).  Graphs that do not fit sw_kernel's shared memory: always.
 bool sw_hooks(const oj_graph* g, int R, int sm_count) {
-  return sw_has_quads(g->n, (size_t)g->sw_ne) && (g->n >= 8192 || (g->n >= 2048 && R <= 2 * sm_count) || (g->n >= 1024 && R <= sm_count));
+  if (!sw_has_quads(g->n, (size_t)g->sw_ne)) return false;
+  if (g->n > sw_max_sites()) return true;
+  if (R <= sm_count) return g->n >= 1024 && g->sw_ne >= 2100;
+  if (!g->local) return g->n >= 40000;
+  return g->n >= 8192 || (R <= 2 * sm_count && g->n >= 2048 && g->sw_ne >= 6500);
 }
 
 }  // namespace

@@ -57,3 +57,21 @@ def test_swendsen_wang_around_the_shared_memory_limits_bit_exact(ctx, side):
     s = s0.copy()
     N.sw_run(dg, s, betas, np.ones(2, np.int32), seed=63)
     np.testing.assert_array_equal(s, O.replay_sw(g, s0, betas.astype(np.float32), 63))
+
+
+@pytest.mark.parametrize("n,bonds,field,R", [(1055, 2100, 0.0, 2), (2055, 6700, 0.0, 149), (8223, 20000, 0.3, 170),
+                                             (8192, 9000, 0.0, 300), (46015, 1, 0.0, 2)])
+def test_swendsen_wang_hooking_near_neighbours_bit_exact(ctx, n, bonds, field, R):
+    """Bonds between sites of near indices, which the hooking kernel takes with
+    several replicas an SM too."""
+    rng = np.random.default_rng(n + bonds)
+    a = rng.integers(0, n - 60, bonds)
+    b = a + rng.integers(1, 60, bonds)
+    h = rng.uniform(-1, 1, n) * (rng.random(n) < field)
+    g = O.AugCSR(I.augmented_from_ising(h, (a, b, rng.normal(size=bonds)), n))
+    dg = N.Graph(ctx, g.n, g.indptr, g.indices, g.data)
+    betas = np.array([0.4, 1.5])
+    s0 = rng.choice(np.array([-1, 1], np.int8), size=(R, n))
+    s = s0.copy()
+    N.sw_run(dg, s, betas, np.ones(2, np.int32), seed=64)
+    np.testing.assert_array_equal(s, O.replay_sw(g, s0, betas.astype(np.float32), 64))

@@ -265,3 +265,26 @@ def test_default_variant_of_large_instances(fake, sizes, reads, variant):
         g = N.Graph(fake.ctx, *I.augmented_csr(I.dense_qubo_int(int(sizes[0]), seed=1)[0]))
         st = N.sa_run(g, np.ones((reads, g.n), np.int8), [1.0], [1], seed=1, kernel="dense_jump")
         assert st["variant"] == variant
+
+
+def _lattice_shuffled(ctx, side):
+    m = I.lattice_pm_j(side, seed=1)[0].tocoo()
+    n = side * side
+    to = np.append(np.random.default_rng(1).permutation(n), n)
+    m.row, m.col = to[m.row], to[m.col]
+    return N.Graph(ctx, *I.augmented_csr(m.tocsr()))
+
+
+@pytest.mark.parametrize("make,R,hooks", [
+    (lambda c: _lattice(c, 32), 148, False), (lambda c: _lattice(c, 33), 148, True), (lambda c: _lattice(c, 33), 149, False),
+    (lambda c: _lattice(c, 56), 256, False), (lambda c: _lattice(c, 64), 296, True), (lambda c: _lattice(c, 64), 297, False),
+    (lambda c: _lattice(c, 91), 1024, True), (lambda c: _lattice_shuffled(c, 91), 148, True),
+    (lambda c: _lattice_shuffled(c, 91), 149, False), (lambda c: _lattice_shuffled(c, 200), 1024, True),
+    (lambda c: _lattice_shuffled(c, 214), 1024, True), (lambda c: _chimera(c, 16), 256, True)])
+def test_default_swendsen_wang_kernel(fake, make, R, hooks):
+    """The hooking kernel runs where it is the faster one, which depends on the
+    bonds, the replicas an SM and the order of the sites."""
+    g = make(fake.ctx)
+    fake.fake_reset()
+    N.sw_run(g, np.ones((R, g.n), np.int8), [1.0], [1], seed=1)
+    assert (b"sw_hook_kernel" in fake.fake_launches()) == hooks
