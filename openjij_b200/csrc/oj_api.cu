@@ -787,8 +787,9 @@ oj_status oj_sa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int8_t* spins, c
         if (Pc == 1 || n / Pc >= 64)
           for (int th : {256, 512, 1024}) cand.push_back(Shape{Pc, th, 0});
       int def_msc = -1;  // the heuristic shape
+      const int def_threads = msc_default_threads(g);
       for (size_t q = 0; q < cand.size(); ++q)
-        if (cand[q].cluster == P && cand[q].threads == msc_default_threads(g, cand[q].cluster)) def_msc = (int)q;
+        if (cand[q].cluster == P && cand[q].threads == def_threads) def_msc = (int)q;
       OJ_CK(ctx->aux.ensure((size_t)G * n * 4), "alloc tuning scratch");
       uint32_t* scratch = ctx->aux.as<uint32_t>();
       const int64_t Ssub = std::min<int64_t>(S, 16);
@@ -809,11 +810,11 @@ oj_status oj_sa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int8_t* spins, c
       tuned_now = true;
     }
     P_used = shp.cluster ? shp.cluster : P;
-    threads_used = shp.threads ? shp.threads : msc_default_threads(g, P_used);
     pe = msc_prepare(g, P_used, &why);
     if (pe != cudaSuccess) {
       return prep_fail(ctx, pe, why);
     }
+    threads_used = shp.threads ? shp.threads : msc_default_threads(g);
     OJ_CK(cudaEventRecord(ctx->ev[1], st), "event");
     if (S > 0)
       OJ_CK(launch_sa_msc(g, G, d_words, d_thr, d_alw, S, rbm, st, &launches, threads_used), "sa bit-packed kernel");

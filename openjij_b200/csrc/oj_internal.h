@@ -78,6 +78,7 @@ struct MscPlan {
   int slots = 0;   // max over parts of nloc + nhalo
   int nlocmax = 0;
   int hmax = 0;
+  int cmax = 0;    // most own sites of one colour class in a part
   DevBuf tables;   // one allocation; the pointers below index into it
   // part-major arrays
   int32_t* gidx = nullptr;   // [P][slots] global site of each slot (-1 = pad)
@@ -145,6 +146,7 @@ struct oj_graph {
   std::vector<int32_t> colour, order, coff;  // greedy colouring; sites sorted by colour
   oj_graph_info info{};
   bool regular = false;
+  bool lumped = false;  // an eighth of the index range holds half of the largest class or more
   bool local = false;  // neighbours' indices differ, on average, by at most n / 16 (counted round the end)
   // device copies
   oj::DevBuf d_rp, d_ci, d_val, d_h, d_val64, d_h64, d_order, d_coff;
@@ -388,7 +390,7 @@ cudaError_t launch_best_slice(const double* energies, int R, int T, int32_t* bes
 
 // Kernel limits used by the planner.
 int msc_max_degree();
-int msc_default_threads(const oj_graph* g, int P);
+int msc_default_threads(const oj_graph* g);  // of the prepared plan
 int cluster_most(int G);
 int split_default_threads(const oj_graph* g, int P);
 int largest_class(const oj_graph* g);

@@ -302,11 +302,13 @@ size_t msc_smem_bytes(const MscPlan& pl) {
 // A thread with at most two sites of a class is bound by the latency of their
 // draws, which then go side by side (lattice of 33 x 33, 1000 sweeps, one CTA per
 // group: 6.5 ms drawn one by one, 4.34 ms); with more sites a thread the draws that
-// a decided site would not have taken cost more (128 x 128 on 4 CTAs).
+// a decided site would not have taken cost more (128 x 128 on 4 CTAs), and so they do
+// in a cluster from seven neighbours on, where more sites of a thread are undecided
+// (one by one / side by side: 8^4 lattice, 520 replicas, 6 CTAs 7.2 / 7.8 us).
 template <int D>
 cudaError_t launch_d(const MscPlan& pl, const MscArgs& a, int G, cudaStream_t st, int threads) {
   const int per_class = (pl.nlocmax + pl.ncol - 1) / pl.ncol;
-  const bool latency = threads <= 512 && per_class <= 2 * threads;
+  const bool latency = threads <= 512 && per_class <= 2 * threads && (pl.P == 1 || D <= 6);
   const bool single = pl.P == 1 && (latency || threads > 512);
   auto kern = threads > 512 ? (single ? sa_msc_kernel<D, kMscMaxThreads, false, 1> : sa_msc_kernel<D, kMscMaxThreads, true, 1>)
                             : (!latency ? sa_msc_kernel<D, 512, true, 1>
@@ -374,17 +376,21 @@ int largest_class(const oj_graph* g) {
 
 // Threads of a CTA: a whole group in one CTA takes one per site of its largest
 // class (8 x 8 lattice: 512 threads 1.46 us a sweep, 64 1.33), above 1024 sites 1024
-// (100 x 100, 4096 replicas: 512 threads 21.8 us, 1024 20.6); a cluster 256 up to
-// two sites a thread (128 x 128 on 16 CTAs: 512 threads 5.15 us, 256 4.84), else 512.
-int msc_default_threads(const oj_graph* g, int P) {
+// (100 x 100, 4096 replicas: 512 threads 21.8 us, 1024 20.6).  A cluster takes 256 where that
+// is a thread for each site of a part's largest class (4000 sites of degree 6, 210 of a
+// class, 400 replicas: 512 threads 14.7, 256 14.4), and up to two sites a thread when few
+// of them are pushed to other parts (128 x 128 on 16 CTAs: 512 threads 5.15 us, 256 4.84;
+// but 2200 sites of degree 4 with up to 275 of a class: 7.5, 10.5; 20 x 20 x 20 on 9 CTAs:
+// 7.4, 8.4); else 512.
+int msc_default_threads(const oj_graph* g) {
   if (const char* env = std::getenv("OJ_MSC_THREADS")) {
     const int v = std::atoi(env);
     if (v >= 32 && v <= kMscMaxThreads && v % 32 == 0) return v;
   }
-  const int per = (largest_class(g) + P - 1) / P;
-  if (P == 1 && per > 1024) return kMscMaxThreads;
-  if (P == 1) return std::max(64, std::min(kMscDefaultThreads, (per + 31) / 32 * 32));
-  return per <= 512 ? 256 : kMscDefaultThreads;
+  const MscPlan& pl = *g->msc;
+  if (pl.P == 1 && pl.cmax > 1024) return kMscMaxThreads;
+  if (pl.P == 1) return std::max(64, std::min(kMscDefaultThreads, (pl.cmax + 31) / 32 * 32));
+  return pl.cmax <= 256 || (pl.cmax <= 512 && 2 * pl.pmax < pl.nlocmax) ? 256 : kMscDefaultThreads;
 }
 
 // The most CTAs a cluster may have for G clusters to run at once: a cluster
@@ -401,7 +407,9 @@ int cluster_most(int G) {
 // Cluster size: the number of CTAs per replica group.  One CTA per SM, as
 // many CTAs as run at once (measured on the L=128 lattice: one 512-thread
 // CTA per SM beats two smaller ones and uneven multi-CTA packings), within the
-// shared-memory budget; a single CTA, whose phases need no cluster barrier, up to
+// shared-memory budget.  Where a colour class is lumped in one part, its size and not
+// the other clusters sets the time, so that more parts win (10000 sites of degree 8 on a
+// ring with far bonds, 400 replicas: 9 CTAs 28.2 us, 11 24.3).  A single CTA, whose phases need no cluster barrier, up to
 // 640 sites a class (us a sweep with one CTA / a cluster, 32 replicas: 45 x 45, four
 // classes of 507 sites, 5.7 / 7.4; 36 x 36, two of 648, 4.0 / 3.7).
 int msc_choose_cluster(const oj_graph* g, int G, int sm_count) {
@@ -414,7 +422,7 @@ int msc_choose_cluster(const oj_graph* g, int G, int sm_count) {
     const size_t per = (size_t)((g->n + P - 1) / P);
     return per * (4 + 6 + 2 * (size_t)D) + per / 2 * 4 <= kMscSmemBytes;
   };
-  int P = std::max(1, std::min(cluster_most(G), sm_count / std::max(G, 1)));
+  int P = std::max(1, std::min(g->lumped ? kMscMaxCluster : cluster_most(G), sm_count / std::max(G, 1)));
   while (P > 1 && g->n / P < 256) --P;
   if (largest_class(g) <= 640) P = 1;
   while (P < kMscMaxCluster && !fits(P)) ++P;
@@ -456,7 +464,7 @@ cudaError_t msc_prepare(oj_graph* g, int P, std::string* why) {
     });
     for (size_t s = 0; s < pt.own.size(); ++s) slot_of[pt.own[s]] = (int)s;
   }
-  int slots = 0, nlocmax = 0, hmax = 0;
+  int slots = 0, nlocmax = 0, hmax = 0, cmax = 0;
   for (int p = 0; p < P; ++p) {
     Part& pt = parts[p];
     std::vector<char> mark(n, 0);
@@ -487,6 +495,7 @@ cudaError_t msc_prepare(oj_graph* g, int P, std::string* why) {
     }
     slots = std::max(slots, (int)(pt.own.size() + pt.halo.size()));
     nlocmax = std::max(nlocmax, (int)pt.own.size());
+    for (int c = 0; c < ncol; ++c) cmax = std::max(cmax, pt.coff[c + 1] - pt.coff[c]);
     hmax = std::max(hmax, (int)pt.halo.size());
   }
   // push lists: every halo slot of every part, filed under the slot of the
@@ -558,6 +567,7 @@ cudaError_t msc_prepare(oj_graph* g, int P, std::string* why) {
   plan->slots = slots;
   plan->nlocmax = nlocmax;
   plan->hmax = hmax;
+  plan->cmax = cmax;
   plan->pmax = pmax;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t b_gidx = al(gidx.size() * 4), b_coff = al(coff.size() * 4), b_cb = al(cbv.size() * 4),
@@ -603,7 +613,7 @@ cudaError_t msc_prepare_from(oj_graph* g, int P, std::string* why) {
 cudaError_t launch_sa_msc(const oj_graph* g, int G, uint32_t* words, const uint32_t* thr,
                           const uint32_t* always, int64_t nsweeps, RngBase rb, cudaStream_t st,
                           int* launches, int threads) {
-  if (threads == 0) threads = msc_default_threads(g, g->msc->P);
+  if (threads == 0) threads = msc_default_threads(g);
   if (threads < 32 || threads > kMscMaxThreads || threads % 32) return cudaErrorInvalidValue;
   const MscPlan& pl = *g->msc;
   MscArgs a;

@@ -288,3 +288,17 @@ def test_default_swendsen_wang_kernel(fake, make, R, hooks):
     fake.fake_reset()
     N.sw_run(g, np.ones((R, g.n), np.int8), [1.0], [1], seed=1)
     assert (b"sw_hook_kernel" in fake.fake_launches()) == hooks
+
+
+@pytest.mark.parametrize("make,R,shape", [
+    (lambda c: _lattice(c, 33), 100, (1, 288)), (lambda c: _lattice(c, 128), 100, (16, 256)),
+    (lambda c: _lattice(c, 128), 400, (9, 512)), (lambda c: _circulant(c, 10000, 8), 400, (11, 512)),
+    (lambda c: _circulant(c, 4000, 4), 100, (15, 512)),
+    (lambda c: N.Graph(c, *I.augmented_csr(I.random_regular_pm_j(10000, 3, seed=4)[0])), 100, (16, 512)),
+    (lambda c: N.Graph(c, *I.augmented_csr(I.random_regular_pm_j(2600, 3, seed=4)[0])), 100, (10, 256))])
+def test_default_shape_of_the_bitpacked_kernel(fake, make, R, shape):
+    """Threads follow the largest class of a part, which on graphs without
+    locality is several times its share."""
+    g = make(fake.ctx)
+    st = N.sa_run(g, np.ones((R, g.n), np.int8), [1.0], [1], seed=1, kernel="bitpacked")
+    assert (st["cluster"], st["threads"]) == shape
