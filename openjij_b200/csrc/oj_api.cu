@@ -1107,7 +1107,7 @@ oj_status oj_sqa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int32_t T, int8
           for (int th : {256, 512}) cand.push_back(Shape{Pc, th, 0});
       int def_split = -1;  // the heuristic shape (the plan prepared above)
       for (size_t q = 0; q < cand.size(); ++q)
-        if (cand[q].cluster == g->msc->P && cand[q].threads == split_default_threads(g, cand[q].cluster)) def_split = (int)q;
+        if (cand[q].cluster == g->msc->P && cand[q].threads == split_default_threads(g, cand[q].cluster, G, ctx->sm_count)) def_split = (int)q;
       OJ_CK(ctx->aux.ensure((size_t)G * 2 * n * 4), "alloc tuning scratch");
       uint32_t* scratch = ctx->aux.as<uint32_t>();
       const int64_t Ssub = std::min<int64_t>(S, 16);
@@ -1134,7 +1134,7 @@ oj_status oj_sqa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int32_t T, int8
       }
     }
     P_used = g->msc->P;
-    threads_used = shp.threads ? shp.threads : split_default_threads(g, P_used);
+    threads_used = shp.threads ? shp.threads : split_default_threads(g, P_used, G, ctx->sm_count);
     if (!pipe) {
       OJ_CK(cudaEventRecord(ctx->ev[1], st), "event");
       if (S > 0)

@@ -272,7 +272,7 @@ bool sqa_split_applies(const oj_graph* g, int T);
 cudaError_t sqa_split_prepare(oj_graph* g, int G, int sm_count, std::string* why, int cluster = 0);
 cudaError_t launch_sqa_split(const oj_graph* g, int G, int T, uint32_t* words, const uint32_t* thr,
                              const uint32_t* mode, int64_t nsweeps, RngBase rb, cudaStream_t st, int* launches,
-                             int threads = 0);
+                             int threads);
 cudaError_t launch_sqa_split_pack(const int8_t* spins, int R, int T, int n, int G, uint32_t* words,
                                   cudaStream_t st);
 cudaError_t launch_sqa_split_unpack(const uint32_t* words, int R, int T, int n, int G, int8_t* spins,
@@ -392,7 +392,7 @@ cudaError_t launch_best_slice(const double* energies, int R, int T, int32_t* bes
 int msc_max_degree();
 int msc_default_threads(const oj_graph* g);  // of the prepared plan
 int cluster_most(int G);
-int split_default_threads(const oj_graph* g, int P);
+int split_default_threads(const oj_graph* g, int P, int G, int sm_count);
 int largest_class(const oj_graph* g);
 cudaError_t msc_prepare(oj_graph* g, int P, std::string* why);
 cudaError_t msc_prepare_from(oj_graph* g, int P, std::string* why);

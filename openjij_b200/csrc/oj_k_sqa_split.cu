@@ -488,16 +488,19 @@ cudaError_t launch_d(const MscPlan& pl, const SplitArgs& a, int G, cudaStream_t 
 
 }  // namespace
 
-// Threads of a CTA: a whole group in one CTA takes one per site of its largest
-// class, but at least 256, which also write the tables (70 sites: 64 threads 5.6 us a
-// sweep, 256 5.1).
-int split_default_threads(const oj_graph* g, int P) {
+// Threads of a CTA: a cluster, and a whole group whose largest class has more than 256
+// sites, 512 (3-regular, 1100 to 1900 sites: within 1 % of one per site).  Smaller ones,
+// which also have a sweep's tables to write, 256 where these are small (degree 3: 70 to
+// 900 sites 1 % less than with 512) or where more groups than SMs share them (lattice of
+// 16 x 16, 32 slices, 1024 replicas: 256 threads 0.71 of the time with 512), else 512 (16 x 16,
+// 16 slices, 64 replicas: 256 threads 10 % more).
+int split_default_threads(const oj_graph* g, int P, int G, int sm_count) {
   if (const char* env = std::getenv("OJ_SQA_THREADS")) {
     const int v = std::atoi(env);
     if (v >= 32 && v <= kSplitMaxThreads && v % 32 == 0) return v;
   }
-  if (P > 1) return kSplitDefaultThreads;
-  return std::max(256, std::min(kSplitDefaultThreads, (largest_class(g) + 31) / 32 * 32));
+  const bool small = P == 1 && largest_class(g) <= 256;
+  return small && (g->info.max_degree == 3 || G > sm_count) ? 256 : kSplitDefaultThreads;
 }
 
 int sqa_split_replicas_per_group(int T) {
@@ -542,7 +545,6 @@ cudaError_t sqa_split_prepare(oj_graph* g, int G, int sm_count, std::string* why
 cudaError_t launch_sqa_split(const oj_graph* g, int G, int T, uint32_t* words, const uint32_t* thr,
                              const uint32_t* mode, int64_t nsweeps, RngBase rb, cudaStream_t st, int* launches,
                              int threads) {
-  if (threads == 0) threads = split_default_threads(g, g->msc->P);
   if (threads < 32 || threads > kSplitMaxThreads || threads % 32) return cudaErrorInvalidValue;
   const MscPlan& pl = *g->msc;
   SplitArgs a;

@@ -302,3 +302,13 @@ def test_default_shape_of_the_bitpacked_kernel(fake, make, R, shape):
     g = make(fake.ctx)
     st = N.sa_run(g, np.ones((R, g.n), np.int8), [1.0], [1], seed=1, kernel="bitpacked")
     assert (st["cluster"], st["threads"]) == shape
+
+
+@pytest.mark.parametrize("make,T,R,threads", [
+    (lambda c: _lattice(c, 16), 16, 64, 512), (lambda c: _lattice(c, 16), 32, 1024, 256),
+    (lambda c: N.Graph(c, *I.augmented_csr(I.random_regular_pm_j(900, 3, seed=4)[0])), 16, 20, 256),
+    (lambda c: N.Graph(c, *I.augmented_csr(I.random_regular_pm_j(1200, 3, seed=4)[0])), 16, 20, 512)])
+def test_default_threads_of_the_slice_split_kernel(fake, make, T, R, threads):
+    g = make(fake.ctx)
+    st = N.sqa_run(g, np.ones((R, T, g.n), np.int8), 1.0, [1.0], [0.5], [1], seed=1, kernel="bitpacked")
+    assert (st["cluster"], st["threads"]) == (1, threads)
