@@ -459,6 +459,15 @@ int time_candidates(cudaStream_t st, int count, Restore restore, Enqueue enqueue
   return bi;
 }
 
+// Index of the default shape among the candidates, to which it is added where it is
+// missing: it is timed like the others and stays unless one of them is clearly faster.
+int with_default(std::vector<Shape>& cand, const Shape& def) {
+  for (size_t q = 0; q < cand.size(); ++q)
+    if (cand[q].cluster == def.cluster && cand[q].threads == def.threads) return (int)q;
+  cand.push_back(def);
+  return (int)cand.size() - 1;
+}
+
 }  // namespace
 
 extern "C" {
@@ -786,10 +795,7 @@ oj_status oj_sa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int8_t* spins, c
       for (int Pc : {1, 2, 4, 8, 16})
         if (Pc == 1 || n / Pc >= 64)
           for (int th : {256, 512, 1024}) cand.push_back(Shape{Pc, th, 0});
-      int def_msc = -1;  // the heuristic shape
-      const int def_threads = msc_default_threads(g);
-      for (size_t q = 0; q < cand.size(); ++q)
-        if (cand[q].cluster == P && cand[q].threads == def_threads) def_msc = (int)q;
+      const int def_msc = with_default(cand, Shape{P, msc_default_threads(g), 0});
       OJ_CK(ctx->aux.ensure((size_t)G * n * 4), "alloc tuning scratch");
       uint32_t* scratch = ctx->aux.as<uint32_t>();
       const int64_t Ssub = std::min<int64_t>(S, 16);
@@ -1105,9 +1111,8 @@ oj_status oj_sqa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int32_t T, int8
       for (int Pc : {1, 2, 4})
         if (Pc == 1 || n / Pc >= 64)
           for (int th : {256, 512}) cand.push_back(Shape{Pc, th, 0});
-      int def_split = -1;  // the heuristic shape (the plan prepared above)
-      for (size_t q = 0; q < cand.size(); ++q)
-        if (cand[q].cluster == g->msc->P && cand[q].threads == split_default_threads(g, cand[q].cluster, G, ctx->sm_count)) def_split = (int)q;
+      const int P0 = g->msc->P;  // the plan prepared above
+      const int def_split = with_default(cand, Shape{P0, split_default_threads(g, P0, G, ctx->sm_count), 0});
       OJ_CK(ctx->aux.ensure((size_t)G * 2 * n * 4), "alloc tuning scratch");
       uint32_t* scratch = ctx->aux.as<uint32_t>();
       const int64_t Ssub = std::min<int64_t>(S, 16);

@@ -312,3 +312,23 @@ def test_default_threads_of_the_slice_split_kernel(fake, make, T, R, threads):
     g = make(fake.ctx)
     st = N.sqa_run(g, np.ones((R, T, g.n), np.int8), 1.0, [1.0], [0.5], [1], seed=1, kernel="bitpacked")
     assert (st["cluster"], st["threads"]) == (1, threads)
+
+
+@pytest.mark.parametrize("make,T,R", [
+    (lambda c: _lattice(c, 8), 0, 64), (lambda c: _lattice(c, 33), 0, 100), (lambda c: _lattice(c, 128), 0, 400),
+    (lambda c: _lattice(c, 32), 0, 256),
+    (lambda c: N.Graph(c, *I.augmented_csr(I.random_regular_pm_j(4096, 3, seed=4)[0])), 16, 8),
+    (lambda c: _lattice(c, 16), 16, 64)])
+def test_the_tuner_times_the_default_shape(fake, make, T, R):
+    """On the stand-in every candidate takes the same time, so a tuned call keeps
+    the untuned one's shape, if that was a candidate at all."""
+    shapes = []
+    for tune in (False, True):
+        g = make(fake.ctx)
+        if T:
+            st = N.sqa_run(g, np.ones((R, T, g.n), np.int8), 1.0, [1.0], [0.5], [4], seed=1, kernel="bitpacked", tune=tune)
+        else:
+            st = N.sa_run(g, np.ones((R, g.n), np.int8), [1.0], [4], seed=1, kernel="bitpacked", tune=tune)
+        assert st["tuned"] == tune
+        shapes.append((st["cluster"], st["threads"]))
+    assert shapes[0] == shapes[1]
