@@ -1680,12 +1680,13 @@ oj_status oj_sa_run_batched(oj_ctx* ctx, const oj_batch* b, const int32_t* reads
   if (count) OJ_CK(cudaMemcpyAsync(d_foff, foff.data(), (size_t)count * 8, cudaMemcpyHostToDevice, st), "H2D offsets");
   bool tuned_now = false;
   if (bm->tuned_variant == 0 && autotune_requested(flags) && S > 0 && nitems > 0) {
-    // the work per sweep follows the acceptance rate, so the candidates run 16
-    // sweeps whose betas are spread over the whole schedule
+    // the work per sweep follows the acceptance rate, so the candidates run up to
+    // 128 sweeps whose betas are spread over the whole schedule, as for one graph: in
+    // 32 the start's many flips weigh too much
     std::vector<int> cand;
     for (int v : {45, 82, 83, 84, 162, 321})
       if (b->max_n <= batch_variant_max_n(v)) cand.push_back(v);
-    const int64_t Ssub = std::min<int64_t>(S, 32);
+    const int64_t Ssub = std::min<int64_t>(S, 128);
     std::vector<float> tb(Ssub);
     for (int64_t q = 0; q < Ssub; ++q) tb[q] = bf[(size_t)((q * S) / Ssub)];
     const size_t sb_al = ((size_t)std::max<int64_t>(sbytes, 16) + 255) & ~(size_t)255;
