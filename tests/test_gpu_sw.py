@@ -65,8 +65,8 @@ def test_swendsen_wang_hooking_near_neighbours_bit_exact(ctx, n, bonds, field, R
     """Bonds between sites of near indices, which the hooking kernel takes with
     several replicas an SM too."""
     rng = np.random.default_rng(n + bonds)
-    a = rng.integers(0, n - 60, bonds)
-    b = a + rng.integers(1, 60, bonds)
+    pair = rng.choice((n - 60) * 60, bonds, replace=False)
+    a, b = pair // 60, pair // 60 + pair % 60 + 1
     h = rng.uniform(-1, 1, n) * (rng.random(n) < field)
     g = O.AugCSR(I.augmented_from_ising(h, (a, b, rng.normal(size=bonds)), n))
     dg = N.Graph(ctx, g.n, g.indptr, g.indices, g.data)
