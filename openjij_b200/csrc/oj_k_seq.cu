@@ -245,8 +245,8 @@ __global__ void __launch_bounds__(2 * kSeqMaxWarps * 32) seq_kernel(SeqArgs a) {
         Sd = Sp + ((size_t)(cd / CPW) * slots + (td & 1)) * sstride + 4 * (cd % CPW) * LP;
       }
       // the next B sites' places in the copy and spins, and this lane's own
-      // site; loaded while the block before is decided, which does not touch
-      // these sites
+      // site; fetched after the block before is decided and stored, so that this
+      // latency is part of every block's chain
       uint32_t* Sb = reinterpret_cast<uint32_t*>(S);
       int o[B];
       uint32_t v[B];
