@@ -41,11 +41,12 @@ namespace {
 constexpr int kSplitMaxThreads = 512;
 constexpr int kSplitDefaultThreads = 512;
 constexpr int kSplitMaxCluster = 16;
-// Philox calls drawn side by side by a CTA with a whole group (3-regular, us a sweep
-// one by one / side by side: 70 sites 5.68 / 5.15, 4096 sites, T = 32, 256 replicas 23.2 /
-// 22.5); in a cluster they only lengthen the work between its barriers (4096 sites,
-// T = 16, 8 replicas: 16.7 / 20.1).
-constexpr int kSplitDraws = 3;
+// Philox calls drawn side by side by a CTA with a whole group (one by one / side by
+// side: 3-regular 70 sites 5.68 / 5.15 us a sweep, 4096 sites, T = 32, 256 replicas 23.2 /
+// 22.5; 4^4 lattice 1.41 to 1; but 16 x 16 lattice 0.92 to 1, 4000 sites of degree 5 or 6 0.96,
+// where the tables' reads already fill the wait); in a cluster they only lengthen the
+// work between its barriers (4096 sites, T = 16, 8 replicas: 16.7 / 20.1).
+constexpr int split_draws(int D) { return D <= 3 || D == 8 ? 3 : 1; }
 constexpr size_t kSplitSmemBytes = 200 * 1024;
 
 struct SplitArgs {
@@ -458,7 +459,7 @@ cudaError_t launch_d(const MscPlan& pl, const SplitArgs& a, int G, cudaStream_t 
   const size_t smem = split_smem_bytes(pl);
   if (smem > kSplitSmemBytes) return cudaErrorInvalidValue;
   if (pl.P == 1) {
-    auto k1 = sqa_split_kernel<D, false, kSplitDraws>;
+    auto k1 = sqa_split_kernel<D, false, split_draws(D)>;
     cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     k1<<<dim3(1, G, 1), threads, smem, st>>>(a);
