@@ -155,6 +155,7 @@ struct oj_graph {
   // the plans of other cluster sizes that earlier calls took: kept, since a run of
   // another context may still read one (at most one for each size)
   std::vector<std::unique_ptr<oj::MscPlan>> msc_other;
+  uint32_t msc_unfit = 0;  // bit P: a partition into P parts does not fit shared memory
   std::unique_ptr<oj::TcPlan> tc;
   oj::DevBuf sqa_nbr, sqa_jm;  // bit-packed SQA tables: [n][D] neighbours (u16), [n] J>0 masks
   std::map<uint64_t, oj::Shape> tuned;  // autotuned launch shapes by (kernel, replicas, slices)

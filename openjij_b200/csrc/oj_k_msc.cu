@@ -437,6 +437,11 @@ cudaError_t msc_prepare(oj_graph* g, int P, std::string* why) {
       std::swap(g->msc, other);
       return cudaSuccess;
     }
+  auto unfit = [&] {
+    if (why) *why = "bit-packed kernel: partition does not fit shared memory; use a larger cluster";
+    return cudaErrorInvalidValue;
+  };
+  if ((g->msc_unfit >> P) & 1u) return unfit();
   const int n = g->n;
   const int D = g->info.max_degree;
   const int ncol = g->info.num_colours;
@@ -514,8 +519,8 @@ cudaError_t msc_prepare(oj_graph* g, int P, std::string* why) {
     pmax = std::max(pmax, (int)push[p].size());
   }
   if (slots > 65535 || (size_t)slots * 4 + (size_t)nlocmax * (6 + 2 * D) + 16 > kMscSmemBytes) {
-    if (why) *why = "bit-packed kernel: partition does not fit shared memory; use a larger cluster";
-    return cudaErrorInvalidValue;
+    g->msc_unfit |= 1u << P;
+    return unfit();
   }
   hmax = std::max(hmax, 1);
   std::vector<int32_t> gidx((size_t)P * slots, 0), coff((size_t)P * (ncol + 1)), cbv((size_t)P * ncol),

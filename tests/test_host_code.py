@@ -332,3 +332,16 @@ def test_the_tuner_times_the_default_shape(fake, make, T, R):
         assert st["tuned"] == tune
         shapes.append((st["cluster"], st["threads"]))
     assert shapes[0] == shapes[1]
+
+
+def test_a_partition_that_does_not_fit_is_tried_once(fake):
+    """Later calls go straight to the cluster that fits: host work between a
+    call's events would count as its time."""
+    g = _circulant(fake.ctx, 40000, 8)
+    s = np.ones((400, g.n), np.int8)
+    N.sa_run(g, s, [1.0], [1], seed=1, kernel="bitpacked")
+    fake.fake_fail_new(0, 64 * 1024)  # a plan's tables are larger
+    N.sa_run(g, s, [1.0], [1], seed=1, kernel="bitpacked", first_sweep=1)
+    pending = fake.fake_new_pending()
+    fake.fake_fail_new(-1, 0)
+    assert pending
