@@ -511,6 +511,7 @@ oj_status oj_ctx_create(int32_t device, oj_ctx** out) {
   }
   ctx->own_stream = true;
   for (auto& e : ctx->ev) cudaEventCreate(&e);
+  active_clusters(ctx->sm_count, ctx->active);
   // set-up of oj_sa_run_bitpacked_noalloc on this device, so that its calls
   // allocate nothing; a failure only disables that entry point
   const cudaError_t pe = noalloc_prepare(device);
@@ -765,7 +766,7 @@ oj_status oj_sa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int8_t* spins, c
     cudaError_t pe = msc_prepare_from(g,
                                       cached != g->tuned.end() && cached->second.cluster
                                           ? cached->second.cluster
-                                          : msc_choose_cluster(g, G, ctx->sm_count),
+                                          : msc_choose_cluster(g, G, ctx->active),
                                       &why);
     if (pe != cudaSuccess) {
       return prep_fail(ctx, pe, why);
@@ -1083,7 +1084,7 @@ oj_status oj_sqa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int32_t T, int8
     const uint64_t key = ((uint64_t)0x80 << 40) | ((uint64_t)T << 32) | (uint64_t)R;
     const auto cached = g->tuned.find(key);
     const cudaError_t pe =
-        sqa_split_prepare(g, G, ctx->sm_count, &why, cached != g->tuned.end() ? cached->second.cluster : 0);
+        sqa_split_prepare(g, G, T, ctx->active, &why, cached != g->tuned.end() ? cached->second.cluster : 0);
     if (pe != cudaSuccess) {
       return prep_fail(ctx, pe, why);
     }
@@ -1122,7 +1123,7 @@ oj_status oj_sqa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int32_t T, int8
           [&] { return cudaMemcpyAsync(scratch, d_words, (size_t)G * 2 * n * 4, cudaMemcpyDeviceToDevice, st); },
           [&](int i) {
             std::string w;
-            const cudaError_t e = sqa_split_prepare(g, G, ctx->sm_count, &w, cand[i].cluster);
+            const cudaError_t e = sqa_split_prepare(g, G, T, ctx->active, &w, cand[i].cluster);
             if (e != cudaSuccess || g->msc->P != cand[i].cluster) return e != cudaSuccess ? e : cudaErrorInvalidValue;
             return launch_sqa_split(g, G, T, scratch, d_thr, d_mode, Ssub, rb, st, nullptr, cand[i].threads);
           },
@@ -1133,7 +1134,7 @@ oj_status oj_sqa_run(oj_ctx* ctx, const oj_graph* gc, int32_t R, int32_t T, int8
       tuned_now = true;
     }
     {
-      const cudaError_t pe2 = sqa_split_prepare(g, G, ctx->sm_count, &why, shp.cluster);
+      const cudaError_t pe2 = sqa_split_prepare(g, G, T, ctx->active, &why, shp.cluster);
       if (pe2 != cudaSuccess) {
         return prep_fail(ctx, pe2, why);
       }

@@ -288,14 +288,6 @@ oj_status finish_graph(oj_ctx* ctx, oj_graph* g) {
         span += std::min(d, n - d);
       }
     g->local = 16.0 * span <= (double)n * (double)g->ci.size();
-    int most = 0, largest = 0;
-    for (int cc = 0; cc < ncol; ++cc) {
-      largest = std::max(largest, g->coff[cc + 1] - g->coff[cc]);
-      std::vector<int> part(8, 0);
-      for (int q = g->coff[cc]; q < g->coff[cc + 1]; ++q)
-        most = std::max(most, ++part[(size_t)((int64_t)g->order[q] * 8 / n)]);
-    }
-    g->lumped = 2 * most >= largest && n > 0;
   }
   // device copies
   cudaError_t e;

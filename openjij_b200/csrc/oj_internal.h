@@ -145,8 +145,8 @@ struct oj_graph {
   std::vector<float> h;
   std::vector<int32_t> colour, order, coff;  // greedy colouring; sites sorted by colour
   oj_graph_info info{};
+  mutable std::atomic<int> part_classes[17] = {};  // see part_class (0: not counted yet)
   bool regular = false;
-  bool lumped = false;  // an eighth of the index range holds half of the largest class or more
   bool local = false;  // neighbours' indices differ, on average, by at most n / 16 (counted round the end)
   // device copies
   oj::DevBuf d_rp, d_ci, d_val, d_h, d_val64, d_h64, d_order, d_coff;
@@ -201,6 +201,7 @@ struct oj_batch {
 struct oj_ctx {
   int device = 0;
   int sm_count = 0;
+  int active[17] = {};  // clusters that run at once (active_clusters)
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   std::string last_error;
@@ -270,7 +271,7 @@ cudaError_t launch_sqa_pack(const int8_t* spins, int R, int T, int n, uint32_t* 
 cudaError_t launch_sqa_unpack(const uint32_t* words, int R, int T, int n, int8_t* spins, cudaStream_t st);
 int sqa_split_replicas_per_group(int T);
 bool sqa_split_applies(const oj_graph* g, int T);
-cudaError_t sqa_split_prepare(oj_graph* g, int G, int sm_count, std::string* why, int cluster = 0);
+cudaError_t sqa_split_prepare(oj_graph* g, int G, int T, const int* active, std::string* why, int cluster = 0);
 cudaError_t launch_sqa_split(const oj_graph* g, int G, int T, uint32_t* words, const uint32_t* thr,
                              const uint32_t* mode, int64_t nsweeps, RngBase rb, cudaStream_t st, int* launches,
                              int threads);
@@ -392,11 +393,12 @@ cudaError_t launch_best_slice(const double* energies, int R, int T, int32_t* bes
 // Kernel limits used by the planner.
 int msc_max_degree();
 int msc_default_threads(const oj_graph* g);  // of the prepared plan
-int cluster_most(int G);
+void active_clusters(int sm_count, int* active);  // [17]: clusters of P CTAs, one CTA an SM, that run at once
 int split_default_threads(const oj_graph* g, int P, int G, int sm_count);
 int largest_class(const oj_graph* g);
+int part_class(const oj_graph* g, int P);  // most sites of a class in one of P parts of the index range
 cudaError_t msc_prepare(oj_graph* g, int P, std::string* why);
 cudaError_t msc_prepare_from(oj_graph* g, int P, std::string* why);
-int msc_choose_cluster(const oj_graph* g, int G, int sm_count);
+int msc_choose_cluster(const oj_graph* g, int G, const int* active);
 
 }  // namespace oj

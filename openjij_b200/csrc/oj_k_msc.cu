@@ -393,26 +393,40 @@ int msc_default_threads(const oj_graph* g) {
   return pl.cmax <= 256 || (pl.cmax <= 512 && 2 * pl.pmax < pl.nlocmax) ? 256 : kMscDefaultThreads;
 }
 
-// The most CTAs a cluster may have for G clusters to run at once: a cluster
-// stays within a GPC, of which a B200 has eight with at least 18 SMs (13 groups of
-// a 128 x 128 lattice: 11 CTAs a cluster, eight clusters at a time, 8.8 us a sweep;
-// 8 CTAs, all at once, 6.3 us).
-int cluster_most(int G) {
-  constexpr int kGpcs = 8, kGpcSms = 18, kMost = 16;
-  int P = kMost;
-  while (P > 1 && kGpcSms / P * kGpcs < G) --P;
-  return P;
+// Most sites of one colour class in one of the P parts that msc_prepare makes;
+// counted once for each P.
+int part_class(const oj_graph* g, int P) {
+  int most = g->part_classes[P].load(std::memory_order_relaxed);
+  if (most > 0) return most;
+  most = 1;
+  for (size_t c = 0; c + 1 < g->coff.size(); ++c) {
+    int p = 0, cnt = 0;  // the sites of a class are in index order
+    for (int q = g->coff[c]; q < g->coff[c + 1]; ++q) {
+      while (g->order[q] >= (int64_t)(p + 1) * g->n / P) {
+        ++p;
+        cnt = 0;
+      }
+      most = std::max(most, ++cnt);
+    }
+  }
+  g->part_classes[P].store(most, std::memory_order_relaxed);
+  return most;
 }
 
-// Cluster size: the number of CTAs per replica group.  One CTA per SM, as
-// many CTAs as run at once (measured on the L=128 lattice: one 512-thread
-// CTA per SM beats two smaller ones and uneven multi-CTA packings), within the
-// shared-memory budget.  Where a colour class is lumped in one part, its size and not
-// the other clusters sets the time, so that more parts win (10000 sites of degree 8 on a
-// ring with far bonds, 400 replicas: 9 CTAs 28.2 us, 11 24.3).  A single CTA, whose phases need no cluster barrier, up to
-// 640 sites a class (us a sweep with one CTA / a cluster, 32 replicas: 45 x 45, four
-// classes of 507 sites, 5.7 / 7.4; 36 x 36, two of 648, 4.0 / 3.7).
-int msc_choose_cluster(const oj_graph* g, int G, int sm_count) {
+// Cluster size: the number of CTAs per replica group, as many as let all groups run at
+// once with a CTA an SM (active, from the driver: a cluster stays within a GPC, so
+// that 22 clusters of 6 run at once but 15 of 7 to 9 and 7 of 11 to 16; us a sweep of a 60-sweep
+// call: 100 x 100 lattice, 8 groups, 16 CTAs 7.2, 10 6.7; 16 groups, 9 CTAs 9.9, 6 7.9; 26
+// groups, 4 CTAs 10.9, 5 8.6).  One group in eight more where CTAs share an SM well, their
+// parts being small or waiting for pushed words (64 x 64, 8 groups: 16 CTAs 5.3, 10 5.5;
+// 3-regular 10000 sites, 16 groups: 9 CTAs 15.8, 6 16.9).  Where a colour class is lumped in
+// one part, its size and not the other clusters sets the time, so that more parts win
+// (10000 sites of degree 8 on a ring with far bonds, 400 replicas: 9 CTAs 28.2 us, 11
+// 24.3).  A single CTA, whose phases need no cluster barrier, up to 640 sites a class (us a
+// sweep with one CTA / a cluster, 32 replicas: 45 x 45, four classes of 507 sites, 5.7 /
+// 7.4; 36 x 36, two of 648, 4.0 / 3.7), 512 where draws take longer (4000 sites of degree 8,
+// classes of 572: 19.0 / 17.3).
+int msc_choose_cluster(const oj_graph* g, int G, const int* active) {
   if (const char* env = std::getenv("OJ_MSC_CLUSTER")) {
     const int v = std::atoi(env);
     if (v >= 1 && v <= kMscMaxCluster) return v;
@@ -422,9 +436,14 @@ int msc_choose_cluster(const oj_graph* g, int G, int sm_count) {
     const size_t per = (size_t)((g->n + P - 1) / P);
     return per * (4 + 6 + 2 * (size_t)D) + per / 2 * 4 <= kMscSmemBytes;
   };
-  int P = std::max(1, std::min(g->lumped ? kMscMaxCluster : cluster_most(G), sm_count / std::max(G, 1)));
+  const int largest = largest_class(g);
+  int P = std::max(1, std::min(kMscMaxCluster, active[1] / std::max(G, 1)));
   while (P > 1 && g->n / P < 256) --P;
-  if (largest_class(g) <= 640) P = 1;
+  if (2 * part_class(g, 8) < largest)
+    while (P > 1 && (active[P] == 0 ||
+                     G > active[P] + (!g->local || g->n / P <= 512 ? std::max(1, active[P] / 8) : 0)))
+      --P;
+  if (largest <= (D <= 6 ? 640 : 512)) P = 1;
   while (P < kMscMaxCluster && !fits(P)) ++P;
   return P;
 }

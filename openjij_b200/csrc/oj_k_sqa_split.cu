@@ -516,18 +516,64 @@ bool sqa_split_applies(const oj_graph* g, int T) {
          T <= 64 && T % 2 == 0;
 }
 
-// Cluster size for G replica groups: one CTA per group, or as many as all run at
-// once (at least 256 sites per CTA) where that is shorter, and a partition whose two
-// halves, halo and tables fit the shared-memory budget.  Time of a phase in us, from
-// 3-regular graphs: one CTA 0.45 + 0.0023 per site of the class; a cluster 2.3 for its
-// barrier and halo (2.8 below 16 CTAs) + 0.0023 per site of a CTA's class (us a sweep, one
-// CTA / a cluster: 1000 sites, T = 4 9.4 / 23.2; 4096 sites, T = 16, 8 replicas 22.2 / 16.1,
-// 64 replicas 22.2 / 23.1).
-cudaError_t sqa_split_prepare(oj_graph* g, int G, int sm_count, std::string* why, int cluster) {
-  int P = std::max(1, std::min(cluster_most(G), sm_count / std::max(G, 1)));
-  while (P > 1 && g->n / P < 256) --P;
-  const double c = largest_class(g);
-  if (0.45 + 0.0023 * c <= (P == kSplitMaxCluster ? 2.3 : 2.8) + 0.0023 * c / P) P = 1;
+// Clusters of P CTAs that run at once, for CTAs that have an SM to themselves: what
+// the driver says for this kernel.
+void active_clusters(int sm_count, int* active) {
+  auto kern = sqa_split_kernel<4, true, 1>;
+  for (int P = 0; P <= kSplitMaxCluster; ++P) active[P] = 0;
+  active[1] = sm_count;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSplitSmemBytes) != cudaSuccess ||
+      cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  for (int P = 2; P <= kSplitMaxCluster; ++P) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(P, 1, 1);
+    cfg.blockDim = dim3(kSplitMaxThreads, 1, 1);
+    cfg.dynamicSmemBytes = kSplitSmemBytes;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = P;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&active[P], kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      active[P] = 0;
+    }
+  }
+}
+
+// Cluster size for G replica groups: one CTA per group, or the most CTAs with which
+// all groups run at once (a second turn costs as much as the first), at least 256
+// sites each, and a partition whose two halves, halo and tables fit the shared-memory
+// budget.  A single CTA where a thread has one site of a class (up to 512; 350 where T is
+// small, so that more draws follow, and neighbours lie in other parts), or where its
+// sweep is estimated shorter, a cluster's being taken 10 % shorter where it has more than
+// two CTAs, because the estimate is short of its gain on small classes.  The estimates (us a
+// sweep) are fits to 788 pairs of graph (rings, 3-regular, square, triangular, cubic and 4-d
+// lattices, ordered and shuffled circulants, degrees 2 to 8) and number of groups, at T = 4 and 32:
+// against the best of all sizes the choice costs 0.7 % on average, 13 % at most
+// but for one; examples (40 sweeps, ms, one CTA / cluster): 3-regular 4096 sites, T = 4, 8 groups
+// 1.18 / 0.79 (10 CTAs), 33 groups 1.21 / 1.11 (4); 4000 sites of degree 5 1.84 / 1.07; 36 x 36
+// 0.67 / 0.56, 74 groups 0.68 / 0.71 (2).
+cudaError_t sqa_split_prepare(oj_graph* g, int G, int T, const int* active, std::string* why, int cluster) {
+  const int c = largest_class(g), D = g->info.max_degree, ph = 2 * g->info.num_colours;
+  int P = kSplitMaxCluster;
+  while (P > 1 && (active[P] < G || g->n / P < 256)) --P;
+  const bool one_fits = (size_t)g->n * (8 + 6 + 2 * D) + 16 <= kSplitSmemBytes;
+  if (c <= (T < 16 && !g->local && D >= 4 && D <= 7 ? 350 : 512)) P = 1;
+  if (P > 1 && one_fits) {
+    struct Fit {
+      double base1, site1, sweep, base, site;  // one CTA: a phase, a site; a cluster: a sweep, a phase, a site
+    };
+    const Fit f = D <= 3 ? Fit{0.5, 0.0030, 4.5, 1.1, 0.0029}
+                         : (D <= 7 ? Fit{0.9, 0.0043, 6.0, 1.2, 0.0040} : Fit{2.2, 0.0075, 6.0, 3.0, 0.0060});
+    const double one = ph * (f.base1 + f.site1 * c), many = f.sweep + ph * (f.base + f.site * part_class(g, P));
+    if (one <= many * (P > 2 ? 0.9 : (T < 16 ? 1.0 : 1.1))) P = 1;
+  }
   if (const char* env = std::getenv("OJ_SQA_CLUSTER")) {
     const int v = std::atoi(env);
     if (v >= 1 && v <= kSplitMaxCluster && v <= g->n) P = v;

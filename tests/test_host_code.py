@@ -292,7 +292,9 @@ def test_default_swendsen_wang_kernel(fake, make, R, hooks):
 
 @pytest.mark.parametrize("make,R,shape", [
     (lambda c: _lattice(c, 33), 100, (1, 288)), (lambda c: _lattice(c, 128), 100, (16, 256)),
-    (lambda c: _lattice(c, 128), 400, (9, 512)), (lambda c: _circulant(c, 10000, 8), 400, (11, 512)),
+    (lambda c: _lattice(c, 128), 256, (10, 512)), (lambda c: _lattice(c, 128), 400, (9, 512)),
+    (lambda c: _lattice(c, 128), 512, (6, 512)), (lambda c: _lattice(c, 128), 832, (5, 512)),
+    (lambda c: _lattice(c, 64), 256, (16, 256)), (lambda c: _circulant(c, 10000, 8), 400, (11, 512)),
     (lambda c: _circulant(c, 4000, 4), 100, (15, 512)),
     (lambda c: N.Graph(c, *I.augmented_csr(I.random_regular_pm_j(10000, 3, seed=4)[0])), 100, (16, 512)),
     (lambda c: N.Graph(c, *I.augmented_csr(I.random_regular_pm_j(2600, 3, seed=4)[0])), 100, (10, 256))])
@@ -332,6 +334,21 @@ def test_the_tuner_times_the_default_shape(fake, make, T, R):
         assert st["tuned"] == tune
         shapes.append((st["cluster"], st["threads"]))
     assert shapes[0] == shapes[1]
+
+
+@pytest.mark.parametrize("make,T,groups,cluster", [
+    (lambda c: _lattice(c, 32), 4, 8, 1), (lambda c: _lattice(c, 36), 4, 8, 5), (lambda c: _lattice(c, 36), 32, 74, 1),
+    (lambda c: N.Graph(c, *I.augmented_csr(I.random_regular_pm_j(4096, 3, seed=4)[0])), 4, 7, 16),
+    (lambda c: N.Graph(c, *I.augmented_csr(I.random_regular_pm_j(4096, 3, seed=4)[0])), 4, 8, 10),
+    (lambda c: N.Graph(c, *I.augmented_csr(I.random_regular_pm_j(4096, 3, seed=4)[0])), 32, 128, 1),
+    (lambda c: _circulant(c, 4000, 6), 32, 22, 6)])
+def test_default_cluster_of_the_slice_split_kernel(fake, make, T, groups, cluster):
+    """A cluster size with which all groups run at once, where that beats one CTA
+    a group."""
+    g = make(fake.ctx)
+    R = groups * {4: 16, 32: 2}[T]
+    st = N.sqa_run(g, np.ones((R, T, g.n), np.int8), 1.0, [1.0], [0.5], [1], seed=1, kernel="bitpacked")
+    assert st["cluster"] == cluster
 
 
 def test_a_partition_that_does_not_fit_is_tried_once(fake):
