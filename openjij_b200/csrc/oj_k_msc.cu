@@ -375,7 +375,9 @@ int largest_class(const oj_graph* g) {
 }
 
 // Threads of a CTA: a whole group in one CTA takes one per site of its largest
-// class (8 x 8 lattice: 512 threads 1.46 us a sweep, 64 1.33), above 1024 sites 1024
+// class (8 x 8 lattice: 512 threads 1.46 us a sweep, 64 1.33), up to 640, so that no class
+// that a cluster would not take (msc_choose_cluster) has a second round for a few sites
+// (47 x 47, classes of 553: 512 threads 7.9 us a sweep, 576 7.2), above 1024 sites 1024
 // (100 x 100, 4096 replicas: 512 threads 21.8 us, 1024 20.6).  A cluster takes 256 where that
 // is a thread for each site of a part's largest class (4000 sites of degree 6, 210 of a
 // class, 400 replicas: 512 threads 14.7, 256 14.4), and up to two sites a thread when few
@@ -389,7 +391,10 @@ int msc_default_threads(const oj_graph* g) {
   }
   const MscPlan& pl = *g->msc;
   if (pl.P == 1 && pl.cmax > 1024) return kMscMaxThreads;
-  if (pl.P == 1) return std::max(64, std::min(kMscDefaultThreads, (pl.cmax + 31) / 32 * 32));
+  if (pl.P == 1) {
+    const int each = std::max(64, (pl.cmax + 31) / 32 * 32);
+    return each <= (pl.D <= 6 ? 640 : kMscDefaultThreads) ? each : kMscDefaultThreads;
+  }
   return pl.cmax <= 256 || (pl.cmax <= 512 && 2 * pl.pmax < pl.nlocmax) ? 256 : kMscDefaultThreads;
 }
 

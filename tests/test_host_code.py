@@ -291,7 +291,8 @@ def test_default_swendsen_wang_kernel(fake, make, R, hooks):
 
 
 @pytest.mark.parametrize("make,R,shape", [
-    (lambda c: _lattice(c, 33), 100, (1, 288)), (lambda c: _lattice(c, 128), 100, (16, 256)),
+    (lambda c: _lattice(c, 33), 100, (1, 288)), (lambda c: _lattice(c, 47), 100, (1, 576)),
+    (lambda c: _lattice(c, 128), 100, (16, 256)),
     (lambda c: _lattice(c, 128), 256, (10, 512)), (lambda c: _lattice(c, 128), 400, (9, 512)),
     (lambda c: _lattice(c, 128), 512, (6, 512)), (lambda c: _lattice(c, 128), 832, (5, 512)),
     (lambda c: _lattice(c, 64), 256, (16, 256)), (lambda c: _circulant(c, 10000, 8), 400, (11, 512)),
