@@ -317,14 +317,16 @@ bool sw_has_quads(int n, size_t ne) { return n < 65535 && sw_hook_smem(n, (ne + 
 // short unless neighbours are near in index order, which makes long chains of sites:
 // from 8192 such sites on, and with two replicas an SM from 2048 sites and 6500 bonds on
 // (lattices with 256 replicas: 46 x 46 13.6 / 15.7, 56 x 56 20.2 / 20.7, 64 x 64 26.2 /
-// 25.0; 1024 replicas: 64 x 64 69 / 71, 91 x 91 152 / 140); without that order only from
+// 25.0; 1024 replicas: 64 x 64 69 / 71, 91 x 91 152 / 140); without that order only with
+// two replicas an SM and four bonds a site from 2048 sites on (random, 256 replicas: 4000 sites
+// of degree 8 43 / 40, 2500 of degree 20 60 / 50; but 4000 of degree 6 33.3 / 33.9), and from
 // 40000 sites on (3-regular, 1024 replicas: 8200 sites 104 / 122, 20000 sites 311 / 332,
 // 40000 sites 941 / 911).  Graphs that do not fit sw_kernel's shared memory: always.
 bool sw_hooks(const oj_graph* g, int R, int sm_count) {
   if (!sw_has_quads(g->n, (size_t)g->sw_ne)) return false;
   if (g->n > sw_max_sites()) return true;
   if (R <= sm_count) return g->n >= 1024 && g->sw_ne >= 2100;
-  if (!g->local) return g->n >= 40000;
+  if (!g->local) return g->n >= 40000 || (R <= 2 * sm_count && g->n >= 2048 && g->sw_ne >= 4 * (int64_t)g->n);
   return g->n >= 8192 || (R <= 2 * sm_count && g->n >= 2048 && g->sw_ne >= 6500);
 }
 
