@@ -551,8 +551,8 @@ void active_clusters(int sm_count, int* active) {
 // sites each, and a partition whose two halves, halo and tables fit the shared-memory
 // budget.  A single CTA where a thread has one site of a class (up to 512; 350 where T is
 // small, so that more draws follow, and neighbours lie in other parts), or where its
-// sweep is estimated shorter, a cluster's being taken 10 % shorter where it has more than
-// two CTAs, because the estimate is short of its gain on small classes.  The estimates (us a
+// sweep is estimated shorter, a cluster's being taken 10 % shorter where it has many
+// CTAs, because the estimate is short of its gain on small classes.  The estimates (us a
 // sweep) are fits to 788 pairs of graph (rings, 3-regular, square, triangular, cubic and 4-d
 // lattices, ordered and shuffled circulants, degrees 2 to 8) and number of groups, at T = 4 and 32:
 // against the best of all sizes the choice costs 0.7 % on average, 13 % at most
@@ -572,7 +572,7 @@ cudaError_t sqa_split_prepare(oj_graph* g, int G, int T, const int* active, std:
     const Fit f = D <= 3 ? Fit{0.5, 0.0030, 4.5, 1.1, 0.0029}
                          : (D <= 7 ? Fit{0.9, 0.0043, 6.0, 1.2, 0.0040} : Fit{2.2, 0.0075, 6.0, 3.0, 0.0060});
     const double one = ph * (f.base1 + f.site1 * c), many = f.sweep + ph * (f.base + f.site * part_class(g, P));
-    if (one <= many * (P > 2 ? 0.9 : (T < 16 ? 1.0 : 1.1))) P = 1;
+    if (one <= many * (P == 2 ? (T < 16 ? 1.0 : 1.1) : (P <= 4 && T >= 16 ? 1.0 : 0.9))) P = 1;
   }
   if (const char* env = std::getenv("OJ_SQA_CLUSTER")) {
     const int v = std::atoi(env);

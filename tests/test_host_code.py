@@ -280,7 +280,9 @@ def _lattice_shuffled(ctx, side):
     (lambda c: _lattice(c, 56), 256, False), (lambda c: _lattice(c, 64), 296, True), (lambda c: _lattice(c, 64), 297, False),
     (lambda c: _lattice(c, 91), 1024, True), (lambda c: _lattice_shuffled(c, 91), 148, True),
     (lambda c: _lattice_shuffled(c, 91), 149, False), (lambda c: _lattice_shuffled(c, 200), 1024, True),
-    (lambda c: _lattice_shuffled(c, 214), 1024, True), (lambda c: _chimera(c, 16), 256, True)])
+    (lambda c: _lattice_shuffled(c, 214), 1024, True), (lambda c: _chimera(c, 16), 256, True),
+    (lambda c: _circulant(c, 4000, 8), 296, True), (lambda c: _circulant(c, 4000, 8), 297, False),
+    (lambda c: _circulant(c, 4000, 6), 296, False)])
 def test_default_swendsen_wang_kernel(fake, make, R, hooks):
     """The hooking kernel runs where it is the faster one, which depends on the
     bonds, the replicas an SM and the order of the sites."""
