@@ -322,8 +322,8 @@ cudaError_t run_batch_enqueue(oj_ctx* ctx, cudaStream_t st, const SweepPlan& p, 
   // Field and sweep kernels that follow one another start early: the field
   // kernel sets up and copies its first digit tiles while the last sweeps finish,
   // and sets the sweep kernel's counter to zero, so that no memset stands between
-  // the two (777 sites, 200 replicas, 500 sweeps 5.70 -> 5.53 ms; 64 instances of 64
-  // to 512 sites 6.35 -> 6.25 ms).  A sweep after the hot-sweep kernel, or the first
+  // the two (777 sites, 200 replicas, 500 sweeps 5.80 -> 5.64 ms; 64 instances of 64
+  // to 512 sites 6.35 -> 6.22 ms).  A sweep after the hot-sweep kernel, or the first
   // one, does not.
   bool early = false;
   int64_t k = 0;
